@@ -1,18 +1,28 @@
 // Flash-attention backward for sm_100a (head_dim 128).
 //
 // One CTA owns one 128-key tile of one (batch, kv-head) and loops over every query head of the group and every
-// query tile that can see those keys.  Per (query tile, key tile) it runs five tcgen05 MMAs:
-//     S  = Q K^T          dP = dO V^T          dV += P^T dO          dK += dS^T Q          dQ_part = dS K
-// with S / dP / dK / dV in the four 128-column quarters of TMEM.  dK and dV stay in TMEM for the whole CTA lifetime
-// (no atomics, GQA heads accumulate in place); the dQ partial is produced in the S columns once S has been consumed
-// and is added to an fp32 scratch tensor with a TMA reduce-add from shared memory (staged in the Q / dO buffers of the
-// iteration, which are idle by then), which a small kernel converts to bf16 at the end.
-// P and dS are formed by 256 threads (two per query row, 64 columns each), written as bf16 to one shared 32 KiB buffer in
-// the 128-byte-swizzled layout the MMAs read (P^T / dS^T as an MN-major A operand, dS as a K-major A operand).
-// Q and dO tiles stream through a 2-stage TMA ring; K and V stay resident in shared memory.
+// query tile that can see those keys.  Scores are kept transposed (TMEM lane = key, column = query), so that P^T goes
+// back to TMEM and is the A operand of its MMA there.  Per (query tile, key tile) five tcgen05 MMAs run:
+//     S^T = K Q^T      dP^T = V dO^T      dV += P^T dO      dQ_part = dS K      dK += dS^T Q
+// TMEM: S^T (P^T over it) | dP^T (dQ_part over it) | dK | dV, 128 columns each.  dK and dV stay in TMEM for the whole
+// CTA lifetime (no atomics, GQA heads accumulate in place).
 //
-// The math is the standard recompute form: P = exp(S - lse), dS = P * (dP - delta) * scale, with
-// delta = rowsum(dO * O) from a pre-pass; a tanh soft-cap multiplies dS by (1 - tanh^2).
+// Roles (16 warps): two compute warpgroups form P and dS (thread <-> key row, 64 query columns), one warpgroup drains the
+// dQ partial to an fp32 scratch tensor with TMA reduce-adds from a staging buffer of its own, and one warpgroup holds
+// the TMA warp, the MMA warp and the warp that brings the row statistics into shared memory.
+//
+// The MMA order is dV(j), S(j+1) | dQ(j), dK(j), dP(j+1): S(j+1) is issued while the compute warps form dS(j), so that
+// P(j+1) is formed under dQ(j) and dK(j); dQ(j) is drained under dK(j); and dS(j+1) is formed under dV(j+1), S(j+2).
+// What bounds it: all MMAs but one take both operands from shared memory (8 KB per 64-cycle instruction, the port's
+// 128 B/clk), and with the staging of dQ and the loads about 512 KB pass the port per tile pair (4100 cycles, against
+// 2560 cycles of tensor work and about 1024 cycles of MUFU work for the exponentials).
+//
+// Forward + backward through the attention op, before (P and dS through shared memory, dQ drained by the compute warps,
+// every MMA waiting for the previous stage of the same tile) and now: B 2, S 4096, H 32 causal 1427 -> 1239 us; B 3,
+// S 1515, H 40 / 8 582 -> 424 us; B 1, S 8192, H 32 / 16, window 4096, soft-cap 2465 -> 1892 us.
+//
+// The math is the standard recompute form: P = exp(S - lse), dS = P * (dP - delta) with the softmax scale applied to the
+// sums dQ and dK, delta = rowsum(dO * O) from a pre-pass; a tanh soft-cap multiplies dS by (1 - tanh^2).
 //
 // Counterpart of the autodiff of `olmax/nn/attention.py:96-103` (cuDNN backward in the reference).
 #include "flash_attn.h"
@@ -31,15 +41,23 @@ constexpr int T = 128;    // tile (queries and keys)
 constexpr int HD = 128;
 constexpr int BLK = 128 * 64 * 2;   // 16 KiB swizzled block [128 rows][64 elems]
 constexpr int TILE = 2 * BLK;       // 32 KiB
-constexpr int STAGES = 2;   // the loops below index stages with (it & 1)
+// Q is needed from S(j) to dK(j), across S(j+1): two stages.  dO is needed for dP(j) and dV(j) only, which are
+// neighbours, and its next tile loads under S(j+1), dQ(j), dK(j): one stage.
 constexpr int OFF_K = 0;
 constexpr int OFF_V = TILE;
-constexpr int OFF_Q = 2 * TILE;                    // STAGES tiles
-constexpr int OFF_DO = OFF_Q + STAGES * TILE;      // STAGES tiles
-constexpr int OFF_P = OFF_DO + STAGES * TILE;      // P, later dS
-constexpr int OFF_BAR = OFF_P + TILE;
-constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-constexpr int THREADS = 352;   // TMA warp, MMA warp, 8 compute warps, dQ store warp
+constexpr int OFF_Q = 2 * TILE;
+constexpr int OFF_DO = 4 * TILE;
+constexpr int OFF_DS = 5 * TILE;                   // dS^T, bf16
+constexpr int OFF_STAGE = 6 * TILE;                // dQ staging: per drain warp two [32 rows][32 floats] slots
+constexpr int SLOT = 32 * 128;
+constexpr int OFF_STATS = OFF_STAGE + 4 * 2 * SLOT;   // [2 stages][-lse * log2(e), -delta][128]
+constexpr int STATS_BYTES = 2 * T * 4;
+constexpr int OFF_BAR = OFF_STATS + 2 * STATS_BYTES;
+constexpr int SMEM_BYTES = OFF_BAR + 256;          // no slack: the base is 1024-byte aligned (checked by the kernel)
+constexpr int THREADS = 512;
+constexpr int COMPUTE_WARPS = 8;
+// registers per thread after the split; 2 * 160 + 96 + 96 = 512 = 4 * the 128 of the launch
+constexpr int REGS_COMPUTE = 160, REGS_DRAIN = 96, REGS_ISSUE = 96;
 constexpr int TMEM_COLS = 512;
 constexpr int C_S = 0, C_DP = 128, C_DK = 256, C_DV = 384;
 
@@ -47,10 +65,10 @@ struct Params {
   int B, S, H, Hkv;
   int Sk, q_off;   // key length; key-axis position of query row 0
   int causal, window;
+  int kv_tiles, group;   // key tiles per slice; (batch, kv-head) slices per scheduling group
   float scale, scale_log2, softcap, scale_over_cap, cap_log2;
   const float* lse;
   const float* delta;
-  float* dq_accum;   // [B, S, H, 128] fp32 contiguous
   bf16* dk; long long dk_sb, dk_ss, dk_sh;
   bf16* dv; long long dv_sb, dv_ss, dv_sh;
   int* status;
@@ -67,34 +85,48 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+template <int N>
+__device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 __global__ void __launch_bounds__(THREADS, 1)
     flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                      const __grid_constant__ CUtensorMap tmDQ, const Params p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint64_t* kv_full = bars + 0;
-  uint64_t* full = bars + 1;       // [STAGES]
-  uint64_t* empty = bars + 3;      // [STAGES]
-  uint64_t* s_full = bars + 5;
-  uint64_t* dp_full = bars + 6;
-  uint64_t* p_ready = bars + 7;    // 8 arrivals (one per compute warp)
-  uint64_t* pv_done = bars + 8;
-  uint64_t* ds_ready = bars + 9;   // 8 arrivals
-  uint64_t* dq_full = bars + 10;
-  uint64_t* dq_read = bars + 11;   // 8 arrivals
-  uint64_t* all_done = bars + 12;
-  uint64_t* dq_staged = bars + 13; // 8 arrivals: the fp32 dQ partial tile is in shared memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* k_full = bars + 0;
+  uint64_t* v_full = bars + 1;
+  uint64_t* q_full = bars + 2;     // [2]
+  uint64_t* q_empty = bars + 4;    // [2]
+  uint64_t* do_full = bars + 6;
+  uint64_t* do_empty = bars + 7;
+  uint64_t* s_full = bars + 8;
+  uint64_t* dp_full = bars + 9;
+  uint64_t* p_ready = bars + 10;   // one arrival per compute warp
+  uint64_t* ds_ready = bars + 11;  // one arrival per compute warp
+  uint64_t* dq_full = bars + 12;
+  uint64_t* dq_read = bars + 13;   // one arrival per drain warp
+  uint64_t* all_done = bars + 14;
+  uint64_t* st_full = bars + 15;   // [2] row statistics
+  uint64_t* st_empty = bars + 17;  // [2] one arrival per compute warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n_tiles = (p.S + T - 1) / T;
-  const int kv_tile = blockIdx.x;
-  const int hkv = blockIdx.y;
-  const int b = blockIdx.z;
+  // Schedule: inside a group of `group` (batch, kv-head) slices the key tiles come in order, all slices of the group for
+  // each tile, so that (causal) the longest loops of the group start first.
+  const int per_group = p.group * p.kv_tiles;
+  const int grp = blockIdx.x / per_group;
+  const int slices = min(p.group, p.B * p.Hkv - grp * p.group);
+  const int in_group = blockIdx.x - grp * per_group;
+  const int kv_tile = in_group / slices;
+  const int bh = grp * p.group + in_group - kv_tile * slices;
+  const int b = bh / p.Hkv;
+  const int hkv = bh - b * p.Hkv;
   const int G = p.H / p.Hkv;
   const int kv0 = kv_tile * T;
 
@@ -106,28 +138,38 @@ __global__ void __launch_bounds__(THREADS, 1)
     i_hi = last < 0 ? -1 : min(i_hi, last / T);
   }
   const int n_q = max(0, i_hi - i_lo + 1);
-  const int n_iters = n_q * G;
+  int n_iters = n_q * G;
+
+  // Swizzled tiles have to start on 1024-byte boundaries.  The kernel has no static shared memory, so its dynamic part
+  // does; were it otherwise, report it and leave the results unwritten (uniform over the CTA: nothing is waited for).
+  if ((smem_u32(smem) & 1023u) != 0) {
+    if (threadIdx.x == 0) report_error(p.status, ERR_BAD_ARG, 699, (int)smem_u32(smem));
+    return;
+  }
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&q_empty[s], 1);
+      mbar_init(&st_full[s], 1);
+      mbar_init(&st_empty[s], COMPUTE_WARPS);
     }
+    mbar_init(do_full, 1);
+    mbar_init(do_empty, 1);
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_ready, 8);     // one arrival per compute warp (lane 0, after the warp has synchronised)
-    mbar_init(pv_done, 1);
-    mbar_init(ds_ready, 8);
+    mbar_init(p_ready, COMPUTE_WARPS);
+    mbar_init(ds_ready, COMPUTE_WARPS);
     mbar_init(dq_full, 1);
-    mbar_init(dq_read, 8);
+    mbar_init(dq_read, 4);
     mbar_init(all_done, 1);
-    mbar_init(dq_staged, 8);
     *abort_flag = 0;
     mbar_fence_init();
     fence_proxy_async();
   }
-  if (warp == 1) {
+  if (warp == 13) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
@@ -136,50 +178,57 @@ __global__ void __launch_bounds__(THREADS, 1)
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  // The TMA, MMA and dQ-store warps run their loops with all 32 lanes so that the loop state stays warp-uniform; one
+  // The issuing and draining warps run their loops with all 32 lanes so that the loop state stays warp-uniform; one
   // elected lane issues.  A wait that gives up marks the warp `dead`: the loop then runs out without issuing anything.
-  if (warp == 0) {
-    const bool leader = elect_one();
-    bool dead = false;
-    if (leader && n_iters > 0) {
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
-      tma_prefetch_desc(&tmDO);
-      mbar_arrive_expect_tx(kv_full, 2 * TILE);
-      tma_load_4d(smem + OFF_K, &tmK, kv_full, 0, hkv, kv0, b);
-      tma_load_4d(smem + OFF_K + BLK, &tmK, kv_full, 64, hkv, kv0, b);
-      tma_load_4d(smem + OFF_V, &tmV, kv_full, 0, hkv, kv0, b);
-      tma_load_4d(smem + OFF_V + BLK, &tmV, kv_full, 64, hkv, kv0, b);
-    }
-    int hq = 0, iq = 0;   // query head within the group, query tile within [i_lo, i_hi]
-    for (int it = 0; it < n_iters; ++it) {
-      const int s = it & 1;
-      const uint32_t ph = (uint32_t)(it >> 1) & 1u;
-      const int h = hkv * G + hq;
-      const int q0 = (i_lo + iq) * T;
-      if (!dead) dead = !mbar_wait(&empty[s], ph ^ 1u, abort_flag, p.status, 700);
-      if (leader && !dead) {
-        mbar_arrive_expect_tx(&full[s], 2 * TILE);
-        uint8_t* sq = smem + OFF_Q + s * TILE;
-        uint8_t* sdo = smem + OFF_DO + s * TILE;
-        tma_load_4d(sq, &tmQ, &full[s], 0, h, q0, b);
-        tma_load_4d(sq + BLK, &tmQ, &full[s], 64, h, q0, b);
-        tma_load_4d(sdo, &tmDO, &full[s], 0, h, q0, b);
-        tma_load_4d(sdo + BLK, &tmDO, &full[s], 64, h, q0, b);
+  if (warp >= 12) {
+    reg_dealloc<REGS_ISSUE>();
+    if (warp == 12) {
+      // ---------------- TMA producer ----------------
+      const bool leader = elect_one();
+      bool dead = false;
+      if (leader && n_iters > 0) {
+        tma_prefetch_desc(&tmQ);
+        tma_prefetch_desc(&tmK);
+        tma_prefetch_desc(&tmV);
+        tma_prefetch_desc(&tmDO);
+        mbar_arrive_expect_tx(k_full, TILE);
+        tma_load_4d(smem + OFF_K, &tmK, k_full, 0, hkv, kv0, b);
+        tma_load_4d(smem + OFF_K + BLK, &tmK, k_full, 64, hkv, kv0, b);
       }
-      if (++iq == n_q) {
-        iq = 0;
-        ++hq;
+      int hq = 0, iq = 0;   // query head within the group, query tile within [i_lo, i_hi]
+      for (int it = 0; it < n_iters; ++it) {
+        const int s = it & 1;
+        const int h = hkv * G + hq;
+        const int q0 = (i_lo + iq) * T;
+        if (!dead) dead = !mbar_wait(&q_empty[s], ((uint32_t)(it >> 1) & 1u) ^ 1u, abort_flag, p.status, 700);
+        if (leader && !dead) {
+          uint8_t* sq = smem + OFF_Q + s * TILE;
+          mbar_arrive_expect_tx(&q_full[s], TILE);
+          tma_load_4d(sq, &tmQ, &q_full[s], 0, h, q0, b);
+          tma_load_4d(sq + BLK, &tmQ, &q_full[s], 64, h, q0, b);
+          if (it == 0) {
+            mbar_arrive_expect_tx(v_full, TILE);
+            tma_load_4d(smem + OFF_V, &tmV, v_full, 0, hkv, kv0, b);
+            tma_load_4d(smem + OFF_V + BLK, &tmV, v_full, 64, hkv, kv0, b);
+          }
+        }
+        if (!dead) dead = !mbar_wait(do_empty, ((uint32_t)it & 1u) ^ 1u, abort_flag, p.status, 701);
+        if (leader && !dead) {
+          mbar_arrive_expect_tx(do_full, TILE);
+          tma_load_4d(smem + OFF_DO, &tmDO, do_full, 0, h, q0, b);
+          tma_load_4d(smem + OFF_DO + BLK, &tmDO, do_full, 64, h, q0, b);
+        }
+        if (++iq == n_q) {
+          iq = 0;
+          ++hq;
+        }
       }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    const bool leader = elect_one();
-    if (n_iters > 0) {
+    } else if (warp == 13 && n_iters > 0) {
+      // ---------------- MMA issue ----------------
+      const bool leader = elect_one();
       constexpr uint32_t id_kk = make_idesc_bf16(T, T, 0, 0);    // both K-major
       constexpr uint32_t id_mm = make_idesc_bf16(T, HD, 1, 1);   // both MN-major
-      constexpr uint32_t id_km = make_idesc_bf16(T, HD, 0, 1);   // A K-major, B MN-major
+      constexpr uint32_t id_km = make_idesc_bf16(T, HD, 0, 1);   // A K-major (or in TMEM), B MN-major
       // Shared-memory descriptors: the high word depends only on the operand's major-ness, the low word is the start
       // address in 16-byte units.  A K-major [128][128] tile is two [128][64] blocks: k step kk sits at
       // (kk / 4) * BLK + (kk % 4) * 32 bytes; in an MN-major tile k step kk sits at kk * 2048 bytes.
@@ -187,100 +236,159 @@ __global__ void __launch_bounds__(THREADS, 1)
       const uint32_t hi_k = (uint32_t)(d_k >> 32), hi_mn = (uint32_t)(d_mn >> 32);
       const uint32_t lo_flags_k = (uint32_t)d_k, lo_flags_mn = (uint32_t)d_mn;   // low-word bits above the address
       auto lo = [](uint32_t addr) { return (addr & 0x3FFFFu) >> 4; };
-      const uint32_t aK = lo(smem_u32(smem + OFF_K)), aV = lo(smem_u32(smem + OFF_V)), aP = lo(smem_u32(smem + OFF_P));
-      const uint32_t aQ0 = lo(smem_u32(smem + OFF_Q)), aDO0 = lo(smem_u32(smem + OFF_DO));
+      const uint32_t aK = lo(smem_u32(smem + OFF_K)), aV = lo(smem_u32(smem + OFF_V)), aDS = lo(smem_u32(smem + OFF_DS));
+      const uint32_t aQ0 = lo(smem_u32(smem + OFF_Q)), aDO = lo(smem_u32(smem + OFF_DO));
       constexpr uint32_t TILE16 = TILE >> 4;
-      bool dead = !mbar_wait(kv_full, 0, abort_flag, p.status, 800);
       auto koff = [](int kk) { return ((uint32_t)(kk >> 2) * BLK + (uint32_t)(kk & 3) * 32) >> 4; };
-      auto issue_s = [&](uint32_t aQ) {
+      auto issue_kk = [&](uint32_t d, uint32_t a, uint32_t bb) {   // D = A B^T over the head dimension
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk)
-          umma_ss_lohi(tmem_base + C_S, lo_flags_k | (aQ + koff(kk)), hi_k, lo_flags_k | (aK + koff(kk)), hi_k, id_kk,
+          umma_ss_lohi(tmem_base + d, lo_flags_k | (a + koff(kk)), hi_k, lo_flags_k | (bb + koff(kk)), hi_k, id_kk,
                        kk != 0 ? 1u : 0u);
       };
-      auto issue_dp = [&](uint32_t aDO) {
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          umma_ss_lohi(tmem_base + C_DP, lo_flags_k | (aDO + koff(kk)), hi_k, lo_flags_k | (aV + koff(kk)), hi_k, id_kk,
-                       kk != 0 ? 1u : 0u);
-      };
-      if (!dead) dead = !mbar_wait(&full[0], 0, abort_flag, p.status, 801);
+      bool dead = !mbar_wait(k_full, 0, abort_flag, p.status, 800);
+      if (!dead) dead = !mbar_wait(&q_full[0], 0, abort_flag, p.status, 801);
       tc_fence_after_sync();
       if (leader && !dead) {
-        issue_s(aQ0);
+        issue_kk(C_S, aK, aQ0);
         umma_commit(s_full);
-        issue_dp(aDO0);
+      }
+      if (!dead) dead = !mbar_wait(v_full, 0, abort_flag, p.status, 802);
+      if (!dead) dead = !mbar_wait(do_full, 0, abort_flag, p.status, 803);
+      tc_fence_after_sync();
+      if (leader && !dead) {
+        issue_kk(C_DP, aV, aDO);
         umma_commit(dp_full);
       }
       for (int it = 0; it < n_iters; ++it) {
-        const int s = it & 1;
-        const uint32_t ph1 = (uint32_t)it & 1u;
-        const uint32_t aQ = aQ0 + (uint32_t)s * TILE16;
-        const uint32_t aDO = aDO0 + (uint32_t)s * TILE16;
-        // dV += P^T dO
-        if (!dead) dead = !mbar_wait(p_ready, ph1, abort_flag, p.status, 802);
+        const uint32_t ph = (uint32_t)it & 1u;
+        const uint32_t aQ = aQ0 + (uint32_t)(it & 1) * TILE16;
+        // dV += P^T dO; P^T of queries [0, 64) is in columns [0, 32) of the S quarter, of the others in [64, 96)
+        if (!dead) dead = !mbar_wait(p_ready, ph, abort_flag, p.status, 804);
         tc_fence_after_sync();
         if (leader && !dead) {
 #pragma unroll
           for (int kk = 0; kk < T / 16; ++kk)
-            umma_ss_lohi(tmem_base + C_DV, lo_flags_mn | (aP + (uint32_t)kk * 128u), hi_mn,
-                         lo_flags_mn | (aDO + (uint32_t)kk * 128u), hi_mn, id_mm, (it | kk) != 0 ? 1u : 0u);
-          umma_commit(pv_done);
+            umma_ts_lohi(tmem_base + C_DV, tmem_base + C_S + (uint32_t)((kk >> 2) * 64 + (kk & 3) * 8),
+                         lo_flags_mn | (aDO + (uint32_t)kk * 128u), hi_mn, id_km, (it | kk) != 0 ? 1u : 0u);
+          umma_commit(do_empty);
         }
-        // dK += dS^T Q ; dQ_part = dS K
-        if (!dead) dead = !mbar_wait(ds_ready, ph1, abort_flag, p.status, 803);
-        tc_fence_after_sync();
-        if (leader && !dead) {
-#pragma unroll
-          for (int kk = 0; kk < T / 16; ++kk)
-            umma_ss_lohi(tmem_base + C_DK, lo_flags_mn | (aP + (uint32_t)kk * 128u), hi_mn,
-                         lo_flags_mn | (aQ + (uint32_t)kk * 128u), hi_mn, id_mm, (it | kk) != 0 ? 1u : 0u);
-#pragma unroll
-          for (int kk = 0; kk < T / 16; ++kk)
-            umma_ss_lohi(tmem_base + C_S, lo_flags_k | (aP + koff(kk)), hi_k, lo_flags_mn | (aK + (uint32_t)kk * 128u), hi_mn,
-                         id_km, kk != 0 ? 1u : 0u);
-          umma_commit(dq_full);   // also tells the compute warps that every MMA reading stage s has finished
-        }
-        if (it + 1 < n_iters) {
+        const bool more = it + 1 < n_iters;
+        if (more) {   // the next scores overwrite P^T: MMAs of one thread run in order
           const int s2 = (it + 1) & 1;
-          const uint32_t ph2 = (uint32_t)((it + 1) >> 1) & 1u;
-          if (!dead) dead = !mbar_wait(&full[s2], ph2, abort_flag, p.status, 804);
+          if (!dead) dead = !mbar_wait(&q_full[s2], (uint32_t)((it + 1) >> 1) & 1u, abort_flag, p.status, 805);
           tc_fence_after_sync();
           if (leader && !dead) {
-            issue_dp(aDO0 + (uint32_t)s2 * TILE16);
-            umma_commit(dp_full);
-          }
-          if (!dead) dead = !mbar_wait(dq_read, ph1, abort_flag, p.status, 805);
-          tc_fence_after_sync();
-          if (leader && !dead) {
-            issue_s(aQ0 + (uint32_t)s2 * TILE16);
+            issue_kk(C_S, aK, aQ0 + (uint32_t)s2 * TILE16);
             umma_commit(s_full);
+          }
+        }
+        // dQ_part = dS K over the dP columns, dK += dS^T Q
+        if (!dead) dead = !mbar_wait(ds_ready, ph, abort_flag, p.status, 806);
+        tc_fence_after_sync();
+        if (leader && !dead) {
+#pragma unroll
+          for (int kk = 0; kk < T / 16; ++kk)
+            umma_ss_lohi(tmem_base + C_DP, lo_flags_mn | (aDS + (uint32_t)kk * 128u), hi_mn,
+                         lo_flags_mn | (aK + (uint32_t)kk * 128u), hi_mn, id_mm, kk != 0 ? 1u : 0u);
+          umma_commit(dq_full);
+#pragma unroll
+          for (int kk = 0; kk < T / 16; ++kk)
+            umma_ss_lohi(tmem_base + C_DK, lo_flags_k | (aDS + koff(kk)), hi_k, lo_flags_mn | (aQ + (uint32_t)kk * 128u),
+                         hi_mn, id_km, (it | kk) != 0 ? 1u : 0u);
+          umma_commit(&q_empty[it & 1]);
+        }
+        if (more) {
+          if (!dead) dead = !mbar_wait(do_full, ph ^ 1u, abort_flag, p.status, 807);
+          if (!dead) dead = !mbar_wait(dq_read, ph, abort_flag, p.status, 808);
+          tc_fence_after_sync();
+          if (leader && !dead) {
+            issue_kk(C_DP, aV, aDO);
+            umma_commit(dp_full);   // all MMAs that read dS(it) have finished too: its buffer may be written again
           }
         }
       }
       if (leader && !dead) umma_commit(all_done);
+    } else if (warp == 14) {
+      // ---------------- row statistics: -lse * log2(e) and -delta of the 128 queries of each iteration ----------------
+      const float LOG2E = 1.4426950408889634f;
+      bool dead = false;
+      int hq = 0, iq = 0;
+      for (int it = 0; it < n_iters; ++it) {
+        const int s = it & 1;
+        const int q0 = (i_lo + iq) * T;
+        const long long base = ((long long)b * p.H + (hkv * G + hq)) * p.S;
+        float l[4], d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {   // rows beyond S: exp2(-inf) = 0
+          const int q = q0 + j * 32 + lane;
+          l[j] = q < p.S ? -__ldg(p.lse + base + q) * LOG2E : -INFINITY;
+          d[j] = q < p.S ? -__ldg(p.delta + base + q) : 0.f;
+        }
+        if (!dead) dead = !mbar_wait(&st_empty[s], ((uint32_t)(it >> 1) & 1u) ^ 1u, abort_flag, p.status, 850);
+        if (!dead) {
+          float* dst = reinterpret_cast<float*>(smem + OFF_STATS + s * STATS_BYTES) + lane;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            dst[j * 32] = l[j];
+            dst[T + j * 32] = d[j];
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&st_full[s]);
+        }
+        if (++iq == n_q) {
+          iq = 0;
+          ++hq;
+        }
+      }
     }
     __syncwarp();
-  } else if (warp == 10) {
-    // ---------------- dQ store warp: fp32 partial tile (in the Q / dO stage) += into global memory ----------------
+  } else if (warp >= 8) {
+    // ---------------- dQ drain: thread <-> query row; fp32 partial += into global memory ----------------
+    reg_dealloc<REGS_DRAIN>();
+    const int qd = warp & 3;
     const bool leader = elect_one();
+    const uint32_t t_src = tmem_base + ((uint32_t)(qd * 32) << 16) + C_DP;
+    uint8_t* slots = smem + OFF_STAGE + qd * 2 * SLOT;
+    const int sw = lane & 7;
     bool dead = false;
     int hq = 0, iq = 0;
-    for (int it = 0; it < n_iters; ++it) {
-      const int s = it & 1;
-      const int h = hkv * G + hq;
-      const int q0 = (i_lo + iq) * T;
-      if (!dead) dead = !mbar_wait(dq_staged, (uint32_t)it & 1u, abort_flag, p.status, 950);
-      if (leader && !dead) {
-        // columns [0, 64) sit in the Q stage, [64, 128) in the dO stage, 32 columns (128 bytes) per chunk
+    auto put = [&](int cc, const uint32_t (&r)[32], int h, int row0) {
+      // at most one copy of this warp may still read its slot: the other slot is free
+      if (leader) tma_store_wait_read<1>();
+      __syncwarp();
+      uint8_t* slot = slots + (cc & 1) * SLOT;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const uint8_t* src = smem + (cc < 2 ? OFF_Q : OFF_DO) + s * TILE + (cc & 1) * 16384;
-          tma_reduce_add_4d(&tmDQ, src, cc * 32, h, q0, b);
-        }
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(slot + lane * 128 + ((j ^ sw) << 4)) =
+            make_uint4(r[j * 4], r[j * 4 + 1], r[j * 4 + 2], r[j * 4 + 3]);
+      fence_proxy_async();
+      __syncwarp();
+      if (leader) {
+        if (row0 < p.S) tma_reduce_add_4d(&tmDQ, slot, cc * 32, h, row0, b);
         tma_store_commit();
-        tma_store_wait_read<0>();      // the stage has been read: hand it back to the TMA producer
-        mbar_arrive(&empty[s]);
+      }
+    };
+    for (int it = 0; it < n_iters; ++it) {
+      const int h = hkv * G + hq;
+      const int row0 = (i_lo + iq) * T + qd * 32;
+      if (!dead) dead = !mbar_wait(dq_full, (uint32_t)it & 1u, abort_flag, p.status, 950);
+      if (!dead) {
+        tc_fence_after_sync();
+        uint32_t r0[32], r1[32];
+        tmem_ld32(t_src, r0);
+        tmem_ld32(t_src + 32, r1);
+        tmem_ld_wait();
+        put(0, r0, h, row0);
+        put(1, r1, h, row0);
+        tmem_ld32(t_src + 64, r0);
+        tmem_ld32(t_src + 96, r1);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dq_read);   // the columns may be overwritten by the next dP
+        put(2, r0, h, row0);
+        put(3, r1, h, row0);
       }
       if (++iq == n_q) {
         iq = 0;
@@ -290,168 +398,151 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (leader) tma_store_wait<0>();
     __syncwarp();
   } else {
-    // ---------------- P / dS / dQ / dK / dV: 8 warps, thread <-> (row, 64-column half) ----------------
+    // ---------------- P / dS: 8 warps, thread <-> (key row, 64 query columns); dK / dV at the end ----------------
     // Two warps share each TMEM lane quarter and split the 128 columns, so that every scheduler has two compute warps
     // to hide TMEM-load, MUFU and shared-memory latencies behind each other.
+    reg_alloc<REGS_COMPUTE>();
     const int qd = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int half = warp >> 2;
     const int row = qd * 32 + lane;
     const int col0 = half * 64;
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16);
-    uint8_t* sP = smem + OFF_P + half * BLK + row * 128;   // this thread's 128-byte row of key block `half`
+    uint8_t* sDS = smem + OFF_DS + half * BLK + row * 128;   // this thread's 128-byte row of query block `half`
     const int sw = row & 7;
-    const float LOG2E = 1.4426950408889634f;
     const bool capped = p.softcap > 0.f;
+    const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+    const int kv_idx = kv0 + row;
+    const bool kv_ok = kv_idx < p.Sk;
     bool ok = true;
-    // Row statistics (log-sum-exp, delta) of the NEXT iteration's query row are fetched one iteration ahead: the loads
-    // (global memory, hundreds of cycles) then complete under the current iteration's work instead of stalling the
-    // exponentials right after S arrives.
-    int hq = 0, iq = 0;          // query head within the group / query tile within [i_lo, i_hi] of iteration `it`
-    // (only the loads are issued ahead; nothing computes on the loaded values until the next iteration, so that no
-    // instruction of this iteration waits for them)
-    float lse_next = INFINITY, dl_next = 0.f;
-    auto fetch_stats = [&](int hq_, int iq_) {
-      const int q_idx_ = min((i_lo + iq_) * T + row, p.S - 1);   // clamped: rows beyond S are masked by q_ok below
-      const long long idx = ((long long)b * p.H + (hkv * G + hq_)) * p.S + q_idx_;
-      lse_next = __ldg(p.lse + idx);
-      dl_next = __ldg(p.delta + idx);
-    };
-    if (n_iters > 0) fetch_stats(0, 0);
+    int iq = 0;
     for (int it = 0; it < n_iters && ok; ++it) {
-      const uint32_t ph1 = (uint32_t)it & 1u;
-      const int q0 = (i_lo + iq) * T;
-      const int q_idx = q0 + row;
-      const bool q_ok = q_idx < p.S;
-      const float lse2 = q_ok ? lse_next * LOG2E : INFINITY;
-      const float dl = q_ok ? dl_next : 0.f;
-      if (++iq == n_q) {
-        iq = 0;
-        ++hq;
-      }
-      if (it + 1 < n_iters) fetch_stats(hq, iq);
-      const int qp0 = p.q_off + q0, q_pos = p.q_off + q_idx;   // positions on the key axis
+      const uint32_t ph = (uint32_t)it & 1u, ph2 = (uint32_t)(it >> 1) & 1u;
+      const int qp0 = p.q_off + (i_lo + iq) * T;   // position of the first query on the key axis
+      if (++iq == n_q) iq = 0;
       const bool need_mask = (kv0 + T > p.Sk) || (p.causal && kv0 + T - 1 > qp0) ||
                              (p.window >= 0 && kv0 < qp0 + T - 1 - p.window);
-      const int kv_hi = p.causal ? min(q_pos, p.Sk - 1) : p.Sk - 1;
-      const int kv_lo = p.window >= 0 ? q_pos - p.window : 0;
+      const float4* st = reinterpret_cast<const float4*>(smem + OFF_STATS + (it & 1) * STATS_BYTES) + half * 16;
 
-      ok = mbar_wait(s_full, ph1, abort_flag, p.status, 900);
+      ok = mbar_wait(&st_full[it & 1], ph2, abort_flag, p.status, 899);
+      if (!ok) break;
+      ok = mbar_wait(s_full, ph, abort_flag, p.status, 900);
       if (!ok) break;
       tc_fence_after_sync();
-      uint32_t pp[32];  // P of this half row, bf16x2
+      uint32_t r0[32], r1[32];   // scores, then P (times 1 - tanh^2 when capped): kept in fp32 until dS is formed
       {
-        uint32_t r0[32], r1[32];
+        uint32_t pp[32];  // P of this half row, bf16x2
         tmem_ld32(t_lane + C_S + (uint32_t)col0, r0);
         tmem_ld32(t_lane + C_S + (uint32_t)(col0 + 32), r1);
         tmem_ld_wait();
         // P = exp2(s * scale * log2e - lse2), in place over the loaded scores.  The soft-cap and mask cases are
         // handled by loops of their own: a branch inside the hot loop would cut it into one basic block per element
         // pair and expose the FFMA -> EX2 -> pack latency of every pair instead of overlapping the pairs.
+        int c_lo = 0, c_hi = T;   // visible columns of this key, relative to col0
+        if (need_mask) {
+          if (p.causal) c_lo = kv_idx - qp0 - col0;
+          if (p.window >= 0) c_hi = kv_idx + p.window - qp0 - col0;
+          if (!kv_ok) c_lo = T;
+        }
         if (capped) {
+          float w0[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            r0[i] = __float_as_uint(fast_exp2(p.cap_log2 * fast_tanh(__uint_as_float(r0[i]) * p.scale_over_cap) - lse2));
-            r1[i] = __float_as_uint(fast_exp2(p.cap_log2 * fast_tanh(__uint_as_float(r1[i]) * p.scale_over_cap) - lse2));
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t(&r)[32] = hh ? r1 : r0;
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 l = st[hh * 8 + (i >> 2)];
+              const float ll[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float t = fast_tanh(__uint_as_float(r[i + j]) * p.scale_over_cap);
+                w0[i + j] = fmaf(-t, t, 1.f);
+                r[i + j] = __float_as_uint(fast_exp2(fmaf(p.cap_log2, t, ll[j])));
+              }
+            }
+            if (need_mask) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (hh * 32 + i < c_lo || hh * 32 + i > c_hi) r[i] = 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              pp[hh * 16 + (i >> 1)] = pack_bf16x2(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+              r[i] = __float_as_uint(__uint_as_float(r[i]) * w0[i]);
+              r[i + 1] = __float_as_uint(__uint_as_float(r[i + 1]) * w0[i + 1]);
+            }
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            r0[i] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(r0[i]), p.scale_log2, -lse2)));
-            r1[i] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(r1[i]), p.scale_log2, -lse2)));
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t(&r)[32] = hh ? r1 : r0;
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 l = st[hh * 8 + (i >> 2)];
+              const float2 a = fma2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, make_float2(l.x, l.y));
+              const float2 c = fma2(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), scale2, make_float2(l.z, l.w));
+              r[i] = __float_as_uint(fast_exp2(a.x));
+              r[i + 1] = __float_as_uint(fast_exp2(a.y));
+              r[i + 2] = __float_as_uint(fast_exp2(c.x));
+              r[i + 3] = __float_as_uint(fast_exp2(c.y));
+            }
+          }
+          if (need_mask) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (i < c_lo || i > c_hi) r0[i] = 0u;
+              if (i + 32 < c_lo || i + 32 > c_hi) r1[i] = 0u;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            pp[i >> 1] = pack_bf16x2(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]));
+            pp[16 + (i >> 1)] = pack_bf16x2(__uint_as_float(r1[i]), __uint_as_float(r1[i + 1]));
           }
         }
-        if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int kv = kv0 + col0 + i;
-            if (kv > kv_hi || kv < kv_lo) r0[i] = 0u;
-            if (kv + 32 > kv_hi || kv + 32 < kv_lo) r1[i] = 0u;
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          pp[i >> 1] = pack_bf16x2(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]));
-          pp[16 + (i >> 1)] = pack_bf16x2(__uint_as_float(r1[i]), __uint_as_float(r1[i + 1]));
-        }
+        // each half keeps to the columns it has read itself: the other half may still be reading its scores
+        tmem_st32(t_lane + C_S + (uint32_t)col0, pp);
+        tmem_st_wait();
       }
-      // eight 16-byte chunks of this row; the chunk index is XOR-swizzled by row % 8 (128-byte swizzle)
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch)
-        *reinterpret_cast<uint4*>(sP + ((ch ^ sw) << 4)) = make_uint4(pp[ch * 4], pp[ch * 4 + 1], pp[ch * 4 + 2], pp[ch * 4 + 3]);
-      fence_proxy_async();
+      tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_ready);
 
-      ok = mbar_wait(dp_full, ph1, abort_flag, p.status, 901);
+      ok = mbar_wait(dp_full, ph, abort_flag, p.status, 901);   // also: the MMAs that read dS(it - 1) have finished
       if (!ok) break;
       tc_fence_after_sync();
-      uint32_t ds[32];
       {
-        uint32_t r0[32], r1[32];
-        tmem_ld32(t_lane + C_DP + (uint32_t)col0, r0);
-        tmem_ld32(t_lane + C_DP + (uint32_t)(col0 + 32), r1);
+        uint32_t g0[32], g1[32];
+        tmem_ld32(t_lane + C_DP + (uint32_t)col0, g0);
+        tmem_ld32(t_lane + C_DP + (uint32_t)(col0 + 32), g1);
         tmem_ld_wait();
+        // eight 16-byte chunks of this row; the chunk index is XOR-swizzled by row % 8 (128-byte swizzle)
 #pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          const float2 pv = unpack_bf16x2(pp[i >> 1]);
-          const float g0 = __uint_as_float(i < 32 ? r0[i] : r1[i - 32]);
-          const float g1 = __uint_as_float(i < 32 ? r0[i + 1] : r1[i - 31]);
-          ds[i >> 1] = pack_bf16x2(pv.x * (g0 - dl) * p.scale, pv.y * (g1 - dl) * p.scale);
+        for (int ch = 0; ch < 8; ++ch) {
+          const uint32_t* g = ch < 4 ? g0 + ch * 8 : g1 + (ch - 4) * 8;
+          const uint32_t* pv = ch < 4 ? r0 + ch * 8 : r1 + (ch - 4) * 8;
+          uint32_t o[4];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float4 dl = st[T / 4 + ch * 2 + j];
+            float2 x = add2(make_float2(__uint_as_float(g[j * 4]), __uint_as_float(g[j * 4 + 1])), make_float2(dl.x, dl.y));
+            float2 y = add2(make_float2(__uint_as_float(g[j * 4 + 2]), __uint_as_float(g[j * 4 + 3])), make_float2(dl.z, dl.w));
+            x = mul2(x, make_float2(__uint_as_float(pv[j * 4]), __uint_as_float(pv[j * 4 + 1])));
+            y = mul2(y, make_float2(__uint_as_float(pv[j * 4 + 2]), __uint_as_float(pv[j * 4 + 3])));
+            o[j * 2] = pack_bf16x2(x.x, x.y);
+            o[j * 2 + 1] = pack_bf16x2(y.x, y.y);
+          }
+          *reinterpret_cast<uint4*>(sDS + ((ch ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
-      if (capped) {  // dS *= 1 - tanh^2 (S is still intact: dQ overwrites it only after ds_ready)
-        uint32_t r0[32], r1[32];
-        tmem_ld32(t_lane + C_S + (uint32_t)col0, r0);
-        tmem_ld32(t_lane + C_S + (uint32_t)(col0 + 32), r1);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          const float t0 = fast_tanh(__uint_as_float(i < 32 ? r0[i] : r1[i - 32]) * p.scale_over_cap);
-          const float t1 = fast_tanh(__uint_as_float(i < 32 ? r0[i + 1] : r1[i - 31]) * p.scale_over_cap);
-          const float2 d = unpack_bf16x2(ds[i >> 1]);
-          ds[i >> 1] = pack_bf16x2(d.x * (1.f - t0 * t0), d.y * (1.f - t1 * t1));
-        }
-      }
-      ok = mbar_wait(pv_done, ph1, abort_flag, p.status, 902);   // dV MMA has consumed P: the buffer may hold dS now
-      if (!ok) break;
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch)
-        *reinterpret_cast<uint4*>(sP + ((ch ^ sw) << 4)) = make_uint4(ds[ch * 4], ds[ch * 4 + 1], ds[ch * 4 + 2], ds[ch * 4 + 3]);
+      tc_fence_before_sync();
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ds_ready);
-
-      ok = mbar_wait(dq_full, ph1, abort_flag, p.status, 903);
-      if (!ok) break;
-      tc_fence_after_sync();
-      // dQ partial: TMEM -> registers -> the (now idle) Q/dO stage as an fp32 [128 x 128] tile made of four
-      // [128 rows][128 B] swizzled chunks; the store warp adds it to global memory with TMA reduce-add.
-      {
-        uint32_t r0[32], r1[32];
-        tmem_ld32(t_lane + C_S + (uint32_t)col0, r0);
-        tmem_ld32(t_lane + C_S + (uint32_t)(col0 + 32), r1);
-        tmem_ld_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dq_read);   // the S / dQ columns may be overwritten by the next S = Q K^T
-        // columns [0, 64) go to this iteration's Q stage, [64, 128) to its dO stage (both idle since dq_full)
-        uint8_t* c0p = (half == 0 ? smem + OFF_Q : smem + OFF_DO) + (it & 1) * TILE;
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          uint8_t* crow = c0p + cc * 16384 + row * 128;
-          const uint32_t* r = cc ? r1 : r0;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(crow + ((j ^ sw) << 4)) = make_uint4(r[j * 4], r[j * 4 + 1], r[j * 4 + 2], r[j * 4 + 3]);
-        }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dq_staged);
+      if (lane == 0) {
+        mbar_arrive(ds_ready);
+        mbar_arrive(&st_empty[it & 1]);
       }
     }
     // dK, dV out (thread <-> key row, 64-column half)
-    const int kv_idx = kv0 + row;
-    const bool kv_ok = kv_idx < p.Sk;
     bf16* dk_row = p.dk + (long long)b * p.dk_sb + (long long)kv_idx * p.dk_ss + (long long)hkv * p.dk_sh + col0;
     bf16* dv_row = p.dv + (long long)b * p.dv_sb + (long long)kv_idx * p.dv_ss + (long long)hkv * p.dv_sh + col0;
     if (n_iters == 0) {
@@ -475,14 +566,13 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               uint4 v, w;
-              v.x = pack_bf16x2(__uint_as_float(r[g * 8 + 0]), __uint_as_float(r[g * 8 + 1]));
-              v.y = pack_bf16x2(__uint_as_float(r[g * 8 + 2]), __uint_as_float(r[g * 8 + 3]));
-              v.z = pack_bf16x2(__uint_as_float(r[g * 8 + 4]), __uint_as_float(r[g * 8 + 5]));
-              v.w = pack_bf16x2(__uint_as_float(r[g * 8 + 6]), __uint_as_float(r[g * 8 + 7]));
-              w.x = pack_bf16x2(__uint_as_float(r2[g * 8 + 0]), __uint_as_float(r2[g * 8 + 1]));
-              w.y = pack_bf16x2(__uint_as_float(r2[g * 8 + 2]), __uint_as_float(r2[g * 8 + 3]));
-              w.z = pack_bf16x2(__uint_as_float(r2[g * 8 + 4]), __uint_as_float(r2[g * 8 + 5]));
-              w.w = pack_bf16x2(__uint_as_float(r2[g * 8 + 6]), __uint_as_float(r2[g * 8 + 7]));
+              uint32_t* vv = reinterpret_cast<uint32_t*>(&v);
+              uint32_t* ww = reinterpret_cast<uint32_t*>(&w);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                vv[j] = pack_bf16x2(__uint_as_float(r[g * 8 + 2 * j]) * p.scale, __uint_as_float(r[g * 8 + 2 * j + 1]) * p.scale);
+                ww[j] = pack_bf16x2(__uint_as_float(r2[g * 8 + 2 * j]), __uint_as_float(r2[g * 8 + 2 * j + 1]));
+              }
               *reinterpret_cast<uint4*>(dk_row + c + g * 8) = v;
               *reinterpret_cast<uint4*>(dv_row + c + g * 8) = w;
             }
@@ -495,13 +585,13 @@ __global__ void __launch_bounds__(THREADS, 1)
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == 13) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]; one warp per (b, s, h) row
+// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d], and the row of the dQ accumulator is cleared; one warp per row
 __global__ void attn_delta_kernel(const bf16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
                                   const bf16* __restrict__ d_o, long long do_sb, long long do_ss, long long do_sh,
-                                  float* __restrict__ delta, int B, int S, int H) {
+                                  float* __restrict__ delta, float* __restrict__ dq_acc, int B, int S, int H) {
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long total = (long long)B * S * H;
@@ -516,11 +606,12 @@ __global__ void attn_delta_kernel(const bf16* __restrict__ o, long long o_sb, lo
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if (lane == 0) delta[((long long)b * H + h) * S + s] = acc;
+  *reinterpret_cast<float4*>(dq_acc + gw * 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// dq[b, s, h, :] (bf16, strided) = dq_accum[b, s, h, :] (fp32 contiguous); one warp per row
+// dq[b, s, h, :] (bf16, strided) = scale * dq_accum[b, s, h, :] (fp32 contiguous); one warp per row
 __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long sb,
-                                       long long ss, long long sh, int B, int S, int H) {
+                                       long long ss, long long sh, float scale, int B, int S, int H) {
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long total = (long long)B * S * H;
@@ -530,16 +621,16 @@ __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __re
   const int b = (int)(gw / ((long long)H * S));
   const float4 v = *reinterpret_cast<const float4*>(acc + gw * 128 + lane * 4);
   uint2 o;
-  o.x = pack_bf16x2(v.x, v.y);
-  o.y = pack_bf16x2(v.z, v.w);
+  o.x = pack_bf16x2(v.x * scale, v.y * scale);
+  o.y = pack_bf16x2(v.z * scale, v.w * scale);
   *reinterpret_cast<uint2*>(dq + b * sb + s * ss + h * sh + lane * 4) = o;
 }
 
-// fp32 dQ accumulator [B, S, H, 128] contiguous -> 4-D map (d, h, s, b), box 32 x 1 x 128 x 1 (128-byte rows)
+// fp32 dQ accumulator [B, S, H, 128] contiguous -> 4-D map (d, h, s, b), box 32 x 1 x 32 x 1 (128-byte rows)
 static int encode_dq_map(CUtensorMap* m, float* acc, int B, int S, int H) {
   uint64_t dims[4] = {128, (uint64_t)H, (uint64_t)S, (uint64_t)B};
   uint64_t str[3] = {128 * 4, (uint64_t)H * 128 * 4, (uint64_t)S * H * 128 * 4};
-  uint32_t box[4] = {32, 1, 128, 1};
+  uint32_t box[4] = {32, 1, 32, 1};
   return encode_tmap(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, acc, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
@@ -549,7 +640,7 @@ static int encode_dq_map(CUtensorMap* m, float* acc, int B, int S, int H) {
 using namespace ob;
 
 // Everything both entry points share: argument checks (all of them before the first enqueue), tensor maps, the delta
-// pre-pass, clearing the dQ accumulator, the main kernel and the fp32 -> bf16 conversion of dQ.  `delta` ([B, H, S]) and
+// pre-pass (which clears the dQ accumulator), the main kernel and the fp32 -> bf16 conversion of dQ.  `delta` ([B, H, S]) and
 // `dq_accum` ([B, S, H, 128], fp32) are the two work buffers, whoever owns them.
 static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, cudaStream_t stream) {
   if (a->D != 128) OB_FAIL(-2, "flash attention kernels are built for head_dim 128 (got %d)", a->D);
@@ -582,10 +673,8 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   const unsigned nblk = (unsigned)((rows + wpb - 1) / wpb);
   fa_bwd::attn_delta_kernel<<<nblk, wpb * 32, 0, stream>>>(
       reinterpret_cast<const bf16*>(a->o), a->o_sb, a->o_ss, a->o_sh, reinterpret_cast<const bf16*>(a->d_o), a->do_sb,
-      a->do_ss, a->do_sh, delta, a->B, a->S, a->H);
+      a->do_ss, a->do_sh, delta, dq_accum, a->B, a->S, a->H);
   OB_CUDA_OK(cudaGetLastError());
-  // the accumulator may hold a previous call's sums: clear the part this call uses
-  OB_CUDA_OK(cudaMemsetAsync(dq_accum, 0, (size_t)rows * 128 * sizeof(float), stream));
 
   fa_bwd::Params p;
   p.B = a->B; p.S = a->S; p.H = a->H; p.Hkv = a->Hkv;
@@ -599,15 +688,19 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   p.cap_log2 = a->softcap * LOG2E;
   p.lse = a->lse;
   p.delta = delta;
-  p.dq_accum = dq_accum;
   p.dk = reinterpret_cast<bf16*>(a->dk); p.dk_sb = a->dk_sb; p.dk_ss = a->dk_ss; p.dk_sh = a->dk_sh;
   p.dv = reinterpret_cast<bf16*>(a->dv); p.dv_sb = a->dv_sb; p.dv_ss = a->dv_ss; p.dv_sh = a->dv_sh;
   p.status = a->status;
-  dim3 grid((Sk + 127) / 128, a->Hkv, a->B);
-  fa_bwd::flash_bwd_kernel<<<grid, fa_bwd::THREADS, fa_bwd::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdq, p);
+  p.kv_tiles = (Sk + 127) / 128;
+  const long long slices = (long long)a->B * a->Hkv, ctas = slices * p.kv_tiles;
+  if (ctas > 0x7fffffffLL) OB_FAIL(-4, "%lld key tiles exceed the grid", ctas);
+  // Few CTAs per SM: the longest loops of all slices first, or the last ones to start set the time.  Many: groups of eight
+  // slices, whose Q / dO / dQ (about 12 MB per 1024 rows and head group of one) stay in L2 while their key tiles run.
+  p.group = ctas <= 4 * 148 ? (int)slices : 8;
+  fa_bwd::flash_bwd_kernel<<<(unsigned)ctas, fa_bwd::THREADS, fa_bwd::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdq, p);
   OB_CUDA_OK(cudaGetLastError());
   fa_bwd::attn_dq_convert_kernel<<<nblk, wpb * 32, 0, stream>>>(dq_accum, reinterpret_cast<bf16*>(a->dq), a->dq_sb,
-                                                               a->dq_ss, a->dq_sh, a->B, a->S, a->H);
+                                                               a->dq_ss, a->dq_sh, a->scale, a->B, a->S, a->H);
   OB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -254,6 +254,31 @@ def test_flash_attention(K, B, S, H, Hkv, causal, window, softcap):
     _check_status()
 
 
+@pytest.mark.parametrize("B,S,H,Hkv,causal,window,softcap", [
+    (1, 8, 2, 1, True, -1, 0.0),          # one partial tile, two heads of a group: two iterations
+    (1, 129, 4, 1, True, -1, 0.0),        # one row and one key beyond a tile; the last dQ drain warps have no rows
+    (2, 257, 3, 3, True, 64, 0.0),        # window narrower than a tile: both diagonal edges cut the same tile
+    (1, 300, 2, 2, True, 130, 25.0),      # window just wider than a tile, with the soft-cap
+    (1, 127, 8, 2, False, -1, 0.0),       # no mask but the sequence's end
+    (4, 640, 16, 8, True, -1, 0.0),       # more key tiles than one scheduling group holds: 160 CTAs, LPT order
+    (2, 1300, 64, 32, True, -1, 0.0),     # 704 CTAs: groups of eight slices
+])
+def test_flash_attention_backward_tile_edges(K, B, S, H, Hkv, causal, window, softcap):
+    """Gradients against fp32 autograd where tiles are cut.  Tolerance: dS, P, the inputs and the result are each rounded
+    to bf16 once (2^-9 relative, independent): about 2 * 2^-9 = 0.4 % in the 2-norm, doubled."""
+    dev = "cuda"
+    torch.manual_seed(13)
+    q, k, v = (torch.randn(B, S, h, 128, device=dev, dtype=torch.bfloat16, requires_grad=True) for h in (H, Hkv, Hkv))
+    o_ref, _ = ref.attention(q.float(), k.float(), v.float(), causal, window, softcap)
+    o, lse = K.flash_attn_fwd(q.detach(), k.detach(), v.detach(), causal=causal, window=window, softcap=softcap)
+    d_o = torch.randn_like(o)
+    want = torch.autograd.grad(o_ref, (q, k, v), d_o.float())
+    got = K.flash_attn_bwd(q.detach(), k.detach(), v.detach(), o, lse, d_o, causal=causal, window=window, softcap=softcap)
+    for g, w in zip(got, want):
+        assert rel_err(g, w) < 8e-3
+    _check_status()
+
+
 @pytest.mark.parametrize("S,Sk,q_off,window,softcap", [
     (256, 512, 256, -1, 0.0),      # late query chunk against the causally visible prefix
     (128, 128, 384, -1, 0.0),      # ring block far below the diagonal: every key visible
