@@ -588,42 +588,102 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == 13) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d], and the row of the dQ accumulator is cleared; one warp per row
-__global__ void attn_delta_kernel(const bf16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
-                                  const bf16* __restrict__ d_o, long long do_sb, long long do_ss, long long do_sh,
-                                  float* __restrict__ delta, float* __restrict__ dq_acc, int B, int S, int H) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long long total = (long long)B * S * H;
-  if (gw >= total) return;
-  const int h = (int)(gw % H);
-  const int s = (int)((gw / H) % S);
-  const int b = (int)(gw / ((long long)H * S));
-  const uint2 a = *reinterpret_cast<const uint2*>(o + b * o_sb + s * o_ss + h * o_sh + lane * 4);
-  const uint2 g = *reinterpret_cast<const uint2*>(d_o + b * do_sb + s * do_ss + h * do_sh + lane * 4);
-  const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), g0 = unpack_bf16x2(g.x), g1 = unpack_bf16x2(g.y);
-  float acc = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) delta[((long long)b * H + h) * S + s] = acc;
-  *reinterpret_cast<float4*>(dq_acc + gw * 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+// Row kernels before and after the main one: 16 lanes per (b, s, h) row, ROWS_PT rows per thread a block's worth apart, all
+// loads of a thread in flight at once.  Bound by HBM: at B 2, S 4096, H 32 one warp per row with 8-byte loads took 58 us
+// (pre-pass) and 48 us (conversion) for 268 and 201 MB; now 38 and 31 us.
+constexpr int ROW_THREADS = 256, ROWS_PT = 4, ROWS_PER_BLOCK = ROW_THREADS / 16 * ROWS_PT;
+
+// 16 bytes of a tensor that no TMA map has checked: in halves where its rows are only 8-byte aligned
+__device__ __forceinline__ uint4 load16(const bf16* p, bool wide) {
+  if (wide) return *reinterpret_cast<const uint4*>(p);
+  const uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 4);
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store16(bf16* p, uint4 v, bool wide) {
+  if (wide) {
+    *reinterpret_cast<uint4*>(p) = v;
+  } else {
+    *reinterpret_cast<uint2*>(p) = make_uint2(v.x, v.y);
+    *reinterpret_cast<uint2*>(p + 4) = make_uint2(v.z, v.w);
+  }
 }
 
-// dq[b, s, h, :] (bf16, strided) = scale * dq_accum[b, s, h, :] (fp32 contiguous); one warp per row
-__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long sb,
-                                       long long ss, long long sh, float scale, int B, int S, int H) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long long total = (long long)B * S * H;
-  if (gw >= total) return;
-  const int h = (int)(gw % H);
-  const int s = (int)((gw / H) % S);
-  const int b = (int)(gw / ((long long)H * S));
-  const float4 v = *reinterpret_cast<const float4*>(acc + gw * 128 + lane * 4);
-  uint2 o;
-  o.x = pack_bf16x2(v.x * scale, v.y * scale);
-  o.y = pack_bf16x2(v.z * scale, v.w * scale);
-  *reinterpret_cast<uint2*>(dq + b * sb + s * ss + h * sh + lane * 4) = o;
+__device__ __forceinline__ void row_coords(unsigned row, int S, int H, int& b, int& s, int& h) {
+  const unsigned bs = row / (unsigned)H;
+  h = (int)(row - bs * (unsigned)H);
+  b = (int)(bs / (unsigned)S);
+  s = (int)(bs - (unsigned)b * (unsigned)S);
+}
+
+// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d], and the row of the dQ accumulator is cleared
+__global__ void __launch_bounds__(ROW_THREADS)
+    attn_delta_kernel(const bf16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
+                      const bf16* __restrict__ d_o, long long do_sb, long long do_ss, long long do_sh,
+                      float* __restrict__ delta, float* __restrict__ dq_acc, int S, int H, unsigned rows, bool wide_o) {
+  const int l16 = threadIdx.x & 15;
+  const unsigned row0 = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 4);
+  int b[ROWS_PT], s[ROWS_PT], h[ROWS_PT];
+  uint4 x[ROWS_PT], g[ROWS_PT];
+#pragma unroll
+  for (int k = 0; k < ROWS_PT; ++k) {
+    const unsigned row = row0 + k * (ROW_THREADS / 16);
+    x[k] = g[k] = make_uint4(0, 0, 0, 0);
+    if (row < rows) {
+      row_coords(row, S, H, b[k], s[k], h[k]);
+      x[k] = load16(o + b[k] * o_sb + s[k] * o_ss + h[k] * o_sh + l16 * 8, wide_o);
+      g[k] = *reinterpret_cast<const uint4*>(d_o + b[k] * do_sb + s[k] * do_ss + h[k] * do_sh + l16 * 8);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < ROWS_PT; ++k) {
+    const unsigned row = row0 + k * (ROW_THREADS / 16);
+    const uint32_t xw[4] = {x[k].x, x[k].y, x[k].z, x[k].w}, gw[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 u = unpack_bf16x2(xw[j]), v = unpack_bf16x2(gw[j]);
+      acc += u.x * v.x + u.y * v.y;
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (row < rows) {
+      if (l16 == 0) delta[((long long)b[k] * H + h[k]) * S + s[k]] = acc;
+      float4* z = reinterpret_cast<float4*>(dq_acc + (long long)row * 128) + l16;
+      z[0] = z[16] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+}
+
+// dq[b, s, h, :] (bf16, strided) = scale * dq_accum[b, s, h, :] (fp32 contiguous)
+__global__ void __launch_bounds__(ROW_THREADS)
+    attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long sb, long long ss, long long sh,
+                           float scale, int S, int H, unsigned rows, bool wide) {
+  const int l16 = threadIdx.x & 15;
+  const unsigned row0 = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 4);
+  float4 v[ROWS_PT][2];
+#pragma unroll
+  for (int k = 0; k < ROWS_PT; ++k) {
+    const unsigned row = row0 + k * (ROW_THREADS / 16);
+    if (row < rows) {
+      const float4* src = reinterpret_cast<const float4*>(acc + (long long)row * 128) + l16 * 2;
+      v[k][0] = src[0];
+      v[k][1] = src[1];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < ROWS_PT; ++k) {
+    const unsigned row = row0 + k * (ROW_THREADS / 16);
+    if (row < rows) {
+      int b, s, h;
+      row_coords(row, S, H, b, s, h);
+      uint4 w;
+      w.x = pack_bf16x2(v[k][0].x * scale, v[k][0].y * scale);
+      w.y = pack_bf16x2(v[k][0].z * scale, v[k][0].w * scale);
+      w.z = pack_bf16x2(v[k][1].x * scale, v[k][1].y * scale);
+      w.w = pack_bf16x2(v[k][1].z * scale, v[k][1].w * scale);
+      store16(dq + b * sb + s * ss + h * sh + l16 * 8, w, wide);
+    }
+  }
 }
 
 // fp32 dQ accumulator [B, S, H, 128] contiguous -> 4-D map (d, h, s, b), box 32 x 1 x 32 x 1 (128-byte rows)
@@ -632,6 +692,10 @@ static int encode_dq_map(CUtensorMap* m, float* acc, int B, int S, int H) {
   uint64_t str[3] = {128 * 4, (uint64_t)H * 128 * 4, (uint64_t)S * H * 128 * 4};
   uint32_t box[4] = {32, 1, 32, 1};
   return encode_tmap(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, acc, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+static bool wide_rows(const void* p, long long sb, long long ss, long long sh) {
+  return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)((sb | ss | sh) * 2)) & 15) == 0;
 }
 
 }  // namespace fa_bwd
@@ -669,11 +733,12 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   }
 
   const long long rows = (long long)a->B * a->S * a->H;
-  const int wpb = 8;  // warps per block
-  const unsigned nblk = (unsigned)((rows + wpb - 1) / wpb);
-  fa_bwd::attn_delta_kernel<<<nblk, wpb * 32, 0, stream>>>(
+  if (rows > 0x7fffffffLL) OB_FAIL(-4, "%lld query rows exceed the index range", rows);
+  const unsigned nblk = (unsigned)((rows + fa_bwd::ROWS_PER_BLOCK - 1) / fa_bwd::ROWS_PER_BLOCK);
+  fa_bwd::attn_delta_kernel<<<nblk, fa_bwd::ROW_THREADS, 0, stream>>>(
       reinterpret_cast<const bf16*>(a->o), a->o_sb, a->o_ss, a->o_sh, reinterpret_cast<const bf16*>(a->d_o), a->do_sb,
-      a->do_ss, a->do_sh, delta, dq_accum, a->B, a->S, a->H);
+      a->do_ss, a->do_sh, delta, dq_accum, a->S, a->H, (unsigned)rows,
+      fa_bwd::wide_rows(a->o, a->o_sb, a->o_ss, a->o_sh));
   OB_CUDA_OK(cudaGetLastError());
 
   fa_bwd::Params p;
@@ -699,8 +764,9 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   p.group = ctas <= 4 * 148 ? (int)slices : 8;
   fa_bwd::flash_bwd_kernel<<<(unsigned)ctas, fa_bwd::THREADS, fa_bwd::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdq, p);
   OB_CUDA_OK(cudaGetLastError());
-  fa_bwd::attn_dq_convert_kernel<<<nblk, wpb * 32, 0, stream>>>(dq_accum, reinterpret_cast<bf16*>(a->dq), a->dq_sb,
-                                                               a->dq_ss, a->dq_sh, a->scale, a->B, a->S, a->H);
+  fa_bwd::attn_dq_convert_kernel<<<nblk, fa_bwd::ROW_THREADS, 0, stream>>>(
+      dq_accum, reinterpret_cast<bf16*>(a->dq), a->dq_sb, a->dq_ss, a->dq_sh, a->scale, a->S, a->H, (unsigned)rows,
+      fa_bwd::wide_rows(a->dq, a->dq_sb, a->dq_ss, a->dq_sh));
   OB_CUDA_OK(cudaGetLastError());
   return 0;
 }

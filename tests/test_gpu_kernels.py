@@ -279,6 +279,25 @@ def test_flash_attention_backward_tile_edges(K, B, S, H, Hkv, causal, window, so
     _check_status()
 
 
+@pytest.mark.parametrize("B,S,H", [(1, 8, 1), (2, 333, 3), (1, 129, 5)])   # rows below, beside and above one block's 64
+def test_flash_attention_backward_with_rows_of_8_byte_alignment(K, B, S, H):
+    """The output and dq may sit in rows that are only 8-byte aligned (no TMA map covers them): same gradients as packed."""
+    torch.manual_seed(17)
+    q, k, v, d_o = (torch.randn(B, S, H, 128, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    o, lse = K.flash_attn_fwd(q, k, v)
+
+    def shifted(t):   # the same values, every row 4 elements into a 132-element slot
+        wide = torch.zeros(B, S, H, 132, device="cuda", dtype=torch.bfloat16)
+        wide[..., 4:] = t
+        return wide[..., 4:]
+
+    want = K.flash_attn_bwd(q, k, v, o, lse, d_o)
+    got = K.flash_attn_bwd(q, k, v, shifted(o), lse, d_o, dq=shifted(torch.zeros_like(q)))
+    for g, w in zip(got, want):
+        assert rel_err(g, w.float()) < 2e-3   # dQ's fp32 sums meet in another order: rounding flips of single bf16 results
+    _check_status()
+
+
 @pytest.mark.parametrize("S,Sk,q_off,window,softcap", [
     (256, 512, 256, -1, 0.0),      # late query chunk against the causally visible prefix
     (128, 128, 384, -1, 0.0),      # ring block far below the diagonal: every key visible
