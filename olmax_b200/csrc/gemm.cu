@@ -480,6 +480,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     const int row_in_tile = q * 32 + lane;
     int it = 0;
+    // chunks staged so far: they alternate between the two buffers across tiles too (a tile clipped at the matrix edge may
+    // have an odd number of them), which is what lets one store still be reading its buffer while the next is filled
+    uint32_t chunk = 0;
     bool ok = true;
     for (int w = worker; w < p.total_items && ok; w += n_workers, ++it) {
       const int buf = it & 1;
@@ -525,7 +528,6 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         const int out_row = (p.c_shard_stride > 0) ? m_local0 : m_shard * p.M_s + m_local0;
         const int out_z = (p.c_shard_stride > 0) ? m_shard : 0;
         const bool store_thread = (threadIdx.x == 64);
-        int chunk = 0;
         for (int c0 = 0; c0 < BN; c0 += cols, ++chunk) {
           if (c0 >= n_valid) break;
           uint8_t* stage_buf = epi_smem + (chunk & 1) * EPI_STAGE_BYTES;

@@ -82,6 +82,21 @@ def test_gemm_cta_pair_tiles_and_split_k_tail(K, M, N, Kd):
     _check_status()
 
 
+@pytest.mark.parametrize("N", [320, 328])   # last column tile of one bf16 chunk: an odd number of staged chunks per tile
+def test_gemm_clipped_tiles_alternate_staging_buffers(K, N):
+    """Many tiles per CTA whose epilogues stage an odd number of chunks: no chunk may be overwritten while it is stored."""
+    torch.manual_seed(23)
+    M, Kd = 148 * 256 * 3, 64
+    a = torch.randn(M, Kd, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, Kd, device="cuda", dtype=torch.bfloat16)
+    c = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+    for _ in range(3):
+        K.gemm(a, b, c, M, N, Kd)
+        err = (c.float() - a.float() @ b.float().t()).abs().amax().item()
+        assert err < 64 * 2 ** -8   # one bf16 rounding of sums of 64 products of unit variance (|c| < 64)
+    _check_status()
+
+
 def test_gemm_sharded_operands(K):
     dev = "cuda"
     torch.manual_seed(1)
