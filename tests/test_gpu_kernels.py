@@ -97,6 +97,31 @@ def test_gemm_clipped_tiles_alternate_staging_buffers(K, N):
     _check_status()
 
 
+@pytest.mark.parametrize("gelu", [False, True])
+@pytest.mark.parametrize("M,h,Kd,keep", [
+    (8, 8, 64, True),            # one partial chunk of one tile
+    (1000, 688, 136, True),      # ragged in every extent; 688 = 5 tiles of 128 and one of 48 columns
+    (296, 192, 1024, False),     # no pre-activations kept
+    (4104, 1416, 64, True),      # several tiles per CTA pair, the last one of 8 columns
+])
+def test_gated_gemm_outputs(K, M, h, Kd, keep, gelu):
+    """act(x Wg^T) * (x Wu^T) and the two pre-activations, each rounded to bf16 once (2^-9 relative, 0.2 % in the 2-norm; the
+    product sees three such roundings)."""
+    torch.manual_seed(M + h)
+    M = M // 8 * 8
+    x = torch.randn(M, Kd, device="cuda", dtype=torch.bfloat16)
+    wg, wu = (torch.randn(h, Kd, device="cuda", dtype=torch.bfloat16) * Kd ** -0.5 for _ in range(2))
+    a, g, u = (torch.full((M, h), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    K.gemm(x, wg, a, M, h, Kd, epi=K.EPI_GEGLU if gelu else K.EPI_SWIGLU, b2=wu, c2=g if keep else None, c3=u if keep else None,
+           ldb=Kd)
+    gr, ur = x.float() @ wg.float().t(), x.float() @ wu.float().t()
+    want = ref.glu(gr, ur, "gelu_tanh" if gelu else "silu")
+    assert rel_err(a, want) < 8e-3
+    if keep:
+        assert rel_err(g, gr) < 4e-3 and rel_err(u, ur) < 4e-3
+    _check_status()
+
+
 def test_gemm_sharded_operands(K):
     dev = "cuda"
     torch.manual_seed(1)
