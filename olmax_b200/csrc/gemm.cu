@@ -11,8 +11,9 @@
 //          drains its own 128 rows from its own TMEM.
 //   CG = 1: one CTA computes a 128 x 256 tile (cta_group::1), four stages; used for problems with too few tiles to
 //          fill the pairs, and selectable for comparison.
-// Accumulating fp32 epilogues (weight gradients) get a split-K tail: the tiles of the last, partly filled wave are
-// cut into k slices so that every SM stays busy; the slices meet in the output through the reduce-add epilogue.
+// Accumulating fp32 epilogues (weight gradients) get a split-K tail: the tiles of the last, partly filled wave (all tiles,
+// where there are fewer than workers) are cut into k slices so that every SM stays busy; the slices meet in the output
+// through the reduce-add epilogue.
 //
 // One kernel covers the three layouts a Linear layer needs (forward Y = X W^T, dgrad dX = dY W, wgrad dW = dY^T X)
 // by letting either operand be K-major or MN-major in shared memory, and covers dim-0-sharded weights by giving
@@ -183,9 +184,11 @@ __device__ __forceinline__ void decode_work(const KernelParams& p, int w, int k_
     k_begin = 0;
     k_count = k_iters;
   } else {
+    // slice by slice, all tiles of the tail for each: what runs at one time reads the same k range of few operand panels
     const int idx = w - p.full_items;
-    tile = p.full_items + idx / p.split;
-    const int sl = idx % p.split;
+    const int tail = (p.total_items - p.full_items) / p.split;
+    tile = p.full_items + idx % tail;
+    const int sl = idx / tail;
     k_begin = (int)((long long)k_iters * sl / p.split);
     k_count = (int)((long long)k_iters * (sl + 1) / p.split) - k_begin;
   }
@@ -888,6 +891,22 @@ static int cta_group_override() {
   }
   return v;
 }
+// Cut `tiles` tiles (fewer than workers) of k_iters iterations into `split` k slices each, dealt to the workers in rounds:
+// the split with the shortest schedule, in iterations.  A slice has at least 16 iterations; every round costs about one
+// more for its epilogue (the reduce-add of an fp32 tile runs under the next slice), the last of them eight.
+struct Split {
+  int split;
+  double cost;
+};
+static Split best_split(int tiles, int workers, int k_iters) {
+  Split best{1, (double)k_iters};
+  for (int s = 2; s <= 64 && k_iters / s >= 16; ++s) {
+    const int rounds = (tiles * s + workers - 1) / workers;
+    const double cost = rounds * ((double)k_iters / s + 1.0) + 8.0;
+    if (cost < 0.98 * best.cost) best = Split{s, cost};
+  }
+  return best;
+}
 static bool split_k_enabled() {
   static int v = -1;
   if (v < 0) {
@@ -923,6 +942,9 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
   kp.n_shards = a->N / N_s;
   kp.k_shards = a->Kc / Kc_s;
   const int cap = a->max_ctas > 0 ? a->max_ctas : sm_count();
+  const int k_iters_total = kp.k_shards * ((Kc_s + BK - 1) / BK);
+  const bool split_ok = split_k_enabled() && !a->no_split_k && a->ag_src == nullptr &&
+                        ((a->epi == EPI_F32_ACC && a->c_shards == nullptr && !a->no_tma_epilogue) || a->epi == EPI_F32_RED);
   // Tile geometry: CTA pairs (256-row tiles) unless forced, or unless the problem has so few 256-row tiles that
   // 128-row tiles on single CTAs keep more SMs busy.
   int CG = cta_group_override();
@@ -1027,23 +1049,16 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
   // slices that meet in the output through reduce-add.
   const int total = kp.m_shards * kp.m_tiles_per_shard * kp.n_shards * kp.n_tiles_per_shard;
   const int max_workers = cap / CG;
-  const int k_iters_total = kp.k_shards * kp.k_iters_per_shard;
   kp.split = 1;
   kp.full_items = total;
   kp.total_items = total;
-  const bool split_ok = split_k_enabled() && !a->no_split_k && a->ag_src == nullptr &&
-                        ((a->epi == EPI_F32_ACC && a->c_shards == nullptr && !a->no_tma_epilogue) || a->epi == EPI_F32_RED);
   if (split_ok) {
     const int rem = total % max_workers;
-    if (rem > 0 && max_workers / rem >= 2) {
-      int split = max_workers / rem;
-      if (split > 8) split = 8;
-      while (split > 1 && k_iters_total / split < 16) --split;
-      if (split > 1) {
-        kp.split = split;
-        kp.full_items = total - rem;
-        kp.total_items = kp.full_items + rem * split;
-      }
+    const int split = rem > 0 ? best_split(rem, max_workers, k_iters_total).split : 1;
+    if (split > 1) {
+      kp.split = split;
+      kp.full_items = total - rem;
+      kp.total_items = kp.full_items + rem * split;
     }
   }
   const int workers = kp.total_items < max_workers ? kp.total_items : max_workers;

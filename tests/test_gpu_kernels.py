@@ -122,6 +122,25 @@ def test_gated_gemm_outputs(K, M, h, Kd, keep, gelu):
     _check_status()
 
 
+@pytest.mark.parametrize("M,N,Kd", [
+    (256, 256, 16 * 64 * 2),         # one tile: two slices of 16 iterations
+    (264, 520, 64 * 64 + 8),         # 2 x 3 ragged tiles, a contraction that ends inside a block
+    (1024, 1024, 40000),             # 16 tiles, dozens of slices, several rounds per worker
+    (5632, 1024, 4096),              # a whole round of tiles, then 14 in slices
+])
+def test_gemm_weight_gradient_in_k_slices(K, M, N, Kd):
+    """The k slices of the tail meet in the fp32 output whatever their number: against fp64, within the error of fp32 sums
+    (each MMA adds 16 products to the accumulator: at most Kd / 16 roundings of 2^-24)."""
+    torch.manual_seed(29)
+    a = torch.randn(Kd, M, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(Kd, N, device="cuda", dtype=torch.bfloat16)
+    c = torch.ones(M, N, device="cuda")
+    K.gemm(a, b, c, M, N, Kd, a_mn=True, b_mn=True, epi=K.EPI_F32_ACC, alpha=0.5)
+    want = 1.0 + 0.5 * (a.double().t() @ b.double())
+    assert ((c.double() - want).norm() / want.norm()).item() < 1e-6 + Kd / 16 * 2 ** -24
+    _check_status()
+
+
 def test_gemm_sharded_operands(K):
     dev = "cuda"
     torch.manual_seed(1)
