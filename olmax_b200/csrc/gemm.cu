@@ -2,15 +2,16 @@
 // CTAs (one per SM), warp-specialised (TMA producer / MMA issuer / 4 epilogue warps), double-buffered accumulators
 // so that the epilogue of tile i overlaps the main loop of tile i+1.
 //
-// Two tile geometries share one kernel body (template parameter CG):
+// The tile geometries share one kernel body (template parameters CG, BN):
 //   CG = 2 (default): a CTA PAIR (2-CTA cluster on the two SMs of a TPC) computes a 256 x 256 tile with
 //          tcgen05.mma.cta_group::2.  Each CTA TMA-loads its own 128 rows of A and its own 128 columns of B per
 //          k-block (32 KiB instead of 48 KiB per 128 x 256 x 64 of work), six stages deep; both CTAs' loads complete on
 //          the leader's mbarrier, the leader's MMA thread issues for the pair and frees the stages / publishes the
 //          accumulator in both CTAs with one tcgen05.commit per CTA (no multicast of any kind).  Each CTA's epilogue
 //          drains its own 128 rows from its own TMEM.
-//   CG = 1: one CTA computes a 128 x 256 tile (cta_group::1), four stages; used for problems with too few tiles to
-//          fill the pairs, and selectable for comparison.
+//   CG = 1: one CTA computes a 128 x 256 tile (cta_group::1), four stages; used for problems with too few tiles to fill
+//          the pairs, and selectable for comparison.  Problems of one wave of 128 x 64 tiles (a prompt or a short
+//          micro-batch through a small model) take those, eight stages deep.
 // Accumulating fp32 epilogues (weight gradients) get a split-K tail: the tiles of the last, partly filled wave (all tiles,
 // where there are fewer than workers) are cut into k slices so that every SM stays busy; the slices meet in the output
 // through the reduce-add epilogue.
@@ -42,24 +43,24 @@
 namespace ob {
 
 constexpr int BM = 128;   // output rows per CTA (the pair tile has CG * BM rows)
-constexpr int BN = 256;   // accumulator columns (MMA N)
+constexpr int BN_WIDE = 256, BN_NARROW = 64;   // accumulator columns (MMA N) of a tile
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int MN_BLOCK_BYTES = 64 * BK * 2;  // one 64(MN) x 64(K) MN-major block: 8 KiB
-constexpr int TMEM_COLS = 512;
 constexpr int GEMM_THREADS = 256;  // warp 0 TMA, 1 MMA, 2-5 epilogue, 6-7 peer-copy (fused all-gather)
 constexpr int COPY_WARPS = 2;
 constexpr int AG_BLOCK_ROWS = 256;  // granularity of the all-gather ready flags
 constexpr int EPI_STAGE_BYTES = 128 * 128;  // one 128-row x 128-byte output chunk
-constexpr int MAX_STAGES = 6;
+constexpr int MAX_STAGES = 8;
 
 // Per-CTA geometry of the two variants: B columns held per CTA, stage size, pipeline depth, shared-memory size.
-template <int CG>
+template <int CG, int BN>
 struct Geo {
   static constexpr int BNL = BN / CG;                    // B columns (rows of the K-major weight) per CTA
-  static constexpr int B_STAGE_BYTES = BNL * BK * 2;     // 32 KiB / 16 KiB
+  static constexpr int B_STAGE_BYTES = BNL * BK * 2;     // 32 KiB / 16 KiB / 8 KiB
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-  static constexpr int STAGES = CG == 1 ? 4 : 6;
+  static constexpr int STAGES = BN == BN_NARROW ? 8 : CG == 1 ? 4 : 6;
+  static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * EPI_STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
 };
 
@@ -68,7 +69,7 @@ struct KernelParams {
   int M_s, N_s, Kc_s;
   int m_tiles_per_shard, n_tiles_per_shard, k_iters_per_shard;
   int m_shards, n_shards, k_shards;
-  int bn_out;  // output columns per tile: 256, or 128 for the gated epilogue
+  int bn_out;  // output columns per tile: BN, or BN / 2 for the gated epilogue
   int epi;
   float alpha;
   void* c;
@@ -194,11 +195,12 @@ __device__ __forceinline__ void decode_work(const KernelParams& p, int w, int k_
   }
 }
 
-template <bool A_MN, bool B_MN, int CG>
+template <bool A_MN, bool B_MN, int CG, int BN>
 __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmB2,
                                           const CUtensorMap& tmC, const CUtensorMap& tmS1, const CUtensorMap& tmS2,
                                           const KernelParams& p) {
-  using G = Geo<CG>;
+  using G = Geo<CG, BN>;
+  constexpr int TMEM_COLS = G::TMEM_COLS;
   constexpr int STAGES = G::STAGES;
   constexpr int STAGE_BYTES = G::STAGE_BYTES;
   constexpr int BNL = G::BNL;
@@ -328,13 +330,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               tma_load_3d(sa, &tmA, &full_bar[stage], k_glob, m0, 0);
             }
             if (B_MN) {
-              // dims (N, Kc_s, k_shards): four 64-wide blocks along N
+              // dims (N, Kc_s, k_shards): BN / 64 64-wide blocks along N
               const int n0 = n_local0;  // MN-major B is never N-sharded
               if (p.b_single) {
                 tma_load_4d(sb, &tmB, &full_bar[stage], 0, k_local, n0 >> 6, k_shard);
               } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < BN / 64; ++j)
                   tma_load_3d(sb + j * MN_BLOCK_BYTES, &tmB, &full_bar[stage], n0 + j * 64, k_local, k_shard);
               }
             } else if (glu) {
@@ -523,7 +525,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         cbase = reinterpret_cast<uint8_t*>(p.c);
         row_off = (long long)(m_shard * p.M_s + m_local0 + row_in_tile) * p.ldc + n_glob0;
       }
-      if (glu && p.tma_epi) {
+      if (BN == BN_WIDE && glu && p.tma_epi) {
         // Gated epilogue, columns [0, 128) = gate, [128, 256) = up: 64 output columns at a time, the activation and (when
         // kept for the backward pass) the two pre-activations staged one after the other and stored by TMA.  With a k loop
         // of 16 iterations this epilogue is longer than the main loop: 65536 x 2816 x 1024 (three outputs) took 898 us with
@@ -661,7 +663,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             }
           }
         }
-      } else if (!glu) {
+      } else if (BN != BN_WIDE || !glu) {
         for (int c0 = 0; c0 < BN; c0 += 32) {
           if (c0 >= n_valid) break;  // warp-uniform
           uint32_t r[32];
@@ -823,12 +825,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   }
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                      const __grid_constant__ CUtensorMap tmS1, const __grid_constant__ CUtensorMap tmS2, const KernelParams p) {
-  gemm_body<A_MN, B_MN, 1>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
+  gemm_body<A_MN, B_MN, 1, BN>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
 }
 
 // The CTA-pair variant: the grid is a whole number of 2-CTA clusters.
@@ -838,7 +840,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                           const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                           const __grid_constant__ CUtensorMap tmS1, const __grid_constant__ CUtensorMap tmS2,
                           const KernelParams p) {
-  gemm_body<A_MN, B_MN, 2>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
+  gemm_body<A_MN, B_MN, 2, BN_WIDE>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
 }
 
 constexpr int MAX_DEVICES = 64;
@@ -848,38 +850,35 @@ struct Maps {
   CUtensorMap A, B, B2, C, S1, S2;
 };
 
-template <bool A_MN, bool B_MN, int CG>
+template <bool A_MN, bool B_MN, int CG, int BN>
 static int launch(const Maps& m, const KernelParams& kp, int grid, cudaStream_t stream) {
   // the shared-memory opt-in is a per-device attribute of the function
   static bool attr_set[MAX_DEVICES] = {};
   int dev = 0;
   OB_CUDA_OK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= MAX_DEVICES) OB_FAIL(-20, "device index %d out of range", dev);
-  if (CG == 2) {
+  constexpr int smem = Geo<CG, BN>::SMEM_BYTES;
+  if constexpr (CG == 2) {
     if (!attr_set[dev]) {
-      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      Geo<2>::SMEM_BYTES));
+      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       attr_set[dev] = true;
     }
-    gemm_bf16_pair_kernel<A_MN, B_MN><<<grid, GEMM_THREADS, Geo<2>::SMEM_BYTES, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
+    gemm_bf16_pair_kernel<A_MN, B_MN><<<grid, GEMM_THREADS, smem, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
   } else {
     if (!attr_set[dev]) {
-      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      Geo<1>::SMEM_BYTES));
+      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       attr_set[dev] = true;
     }
-    gemm_bf16_kernel<A_MN, B_MN><<<grid, GEMM_THREADS, Geo<1>::SMEM_BYTES, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
+    gemm_bf16_kernel<A_MN, B_MN, BN><<<grid, GEMM_THREADS, smem, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
   }
   OB_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-template <int CG>
+template <int CG, int BN>
 static int launch_layout(bool a_mn, bool b_mn, const Maps& m, const KernelParams& kp, int grid, cudaStream_t stream) {
-  if (a_mn) return b_mn ? launch<true, true, CG>(m, kp, grid, stream)
-                        : launch<true, false, CG>(m, kp, grid, stream);
-  return b_mn ? launch<false, true, CG>(m, kp, grid, stream)
-              : launch<false, false, CG>(m, kp, grid, stream);
+  if (a_mn) return b_mn ? launch<true, true, CG, BN>(m, kp, grid, stream) : launch<true, false, CG, BN>(m, kp, grid, stream);
+  return b_mn ? launch<false, true, CG, BN>(m, kp, grid, stream) : launch<false, false, CG, BN>(m, kp, grid, stream);
 }
 
 // 1: force single-CTA tiles, 2: force CTA pairs, 0: choose per problem (OLMAX_B200_GEMM_CTA_GROUP)
@@ -937,7 +936,6 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
   KernelParams kp;
   kp.M = a->M; kp.N = a->N; kp.Kc = a->Kc;
   kp.M_s = M_s; kp.N_s = N_s; kp.Kc_s = Kc_s;
-  kp.bn_out = glu ? 128 : BN;
   kp.m_shards = a->M / M_s;
   kp.n_shards = a->N / N_s;
   kp.k_shards = a->Kc / Kc_s;
@@ -945,19 +943,35 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
   const int k_iters_total = kp.k_shards * ((Kc_s + BK - 1) / BK);
   const bool split_ok = split_k_enabled() && !a->no_split_k && a->ag_src == nullptr &&
                         ((a->epi == EPI_F32_ACC && a->c_shards == nullptr && !a->no_tma_epilogue) || a->epi == EPI_F32_RED);
-  // Tile geometry: CTA pairs (256-row tiles) unless forced, or unless the problem has so few 256-row tiles that
-  // 128-row tiles on single CTAs keep more SMs busy.
+  // Tile geometry: CTA pairs (256-row tiles) unless forced, or unless there are so few 256-row tiles that 128-row tiles on
+  // single CTAs keep more SMs busy (unsharded problems: and the contraction is short).
+  const bool sharded = kp.m_shards * kp.n_shards * kp.k_shards > 1 || a->c_shards != nullptr;
   int CG = cta_group_override();
+  int BN = BN_WIDE;
   if (CG == 0) {
-    const long long n_t = (long long)kp.n_shards * ((N_s + kp.bn_out - 1) / kp.bn_out);
-    const long long pair_tiles = (long long)kp.m_shards * ((M_s + 2 * BM - 1) / (2 * BM)) * n_t;
-    const long long single_tiles = (long long)kp.m_shards * ((M_s + BM - 1) / BM) * n_t;
-    CG = (pair_tiles >= cap / 2 || single_tiles == pair_tiles) ? 2 : 1;
+    auto tiles = [&](int rows, int bn) {
+      const int cols = glu ? bn / 2 : bn;
+      return (long long)kp.m_shards * ((M_s + rows - 1) / rows) * kp.n_shards * ((N_s + cols - 1) / cols);
+    };
+    const long long pair_tiles = tiles(2 * BM, BN_WIDE), single_tiles = tiles(BM, BN_WIDE);
+    // (a k-block takes a pair 277 ns and a single CTA, whose loads bound it, 370; single CTAs start about 1.5 us sooner)
+    CG = (pair_tiles >= cap / 2 || single_tiles == pair_tiles || (!sharded && k_iters_total >= 32)) ? 2 : 1;
     // row shards of at most 128 rows (e.g. the k / v weight gradients of a grouped-query model over 8 GPUs): the
     // second CTA of every pair would have no rows at all
     if (kp.m_shards > 1 && M_s <= BM) CG = 1;
+    // 128 x 64 tiles, where all of them run at once and most pairs would have no 256 x 256 tile.  Their k-blocks come at the
+    // same pace (about 280 ns, bound by the latency of the loads through eight stages), but they start and drain sooner:
+    // 328 x 1024 x 2816 20.5 us against 26.7 with 128 x 256 single-CTA tiles, 1000 x 1024 x 5632 35 against 43, 1024 x
+    // 512 x 512 12.3 against 14.3.  In more than one wave they lose (2048 x 1024 x 50304: 533 us against @LM@ with pairs),
+    // and to k slices on pairs where the contraction is long enough to be cut.
+    if (!sharded && !glu && tiles(BM, BN_WIDE) <= cap / 2 && tiles(BM, BN_NARROW) <= cap &&
+        !(split_ok && best_split((int)pair_tiles, cap / 2, k_iters_total).split > 1)) {
+      CG = 1;
+      BN = BN_NARROW;
+    }
   }
   if (cap < 2) CG = 1;
+  kp.bn_out = glu ? BN / 2 : BN;
   const int BMT = BM * CG;            // tile rows
   const int BNL = BN / CG;            // B columns held per CTA
   kp.m_tiles_per_shard = (M_s + BMT - 1) / BMT;
@@ -1035,7 +1049,7 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     uint64_t dims[3] = {(uint64_t)a->Kc, (uint64_t)N_s, (uint64_t)kp.n_shards};
     uint64_t sstride = kp.n_shards > 1 ? (uint64_t)bss * 2 : (uint64_t)a->ldb * 2 * (uint64_t)N_s;
     uint64_t str[2] = {(uint64_t)a->ldb * 2, sstride};
-    uint32_t box[3] = {(uint32_t)BK, (uint32_t)(glu ? 128 : BNL), 1};
+    uint32_t box[3] = {(uint32_t)BK, (uint32_t)(glu ? BN / 2 : BNL), 1};
     rc = encode_tmap(&tB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->b, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     if (glu) {
@@ -1116,9 +1130,9 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
   if (tma_ok) {
     const bool f32 = a->epi == EPI_F32 || a->epi == EPI_F32_ACC;
     const uint64_t es = f32 ? 4 : 2;
-    const bool sharded = a->c_shard_stride > 0;
-    uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)(sharded ? M_s : a->M), (uint64_t)(sharded ? kp.m_shards : 1)};
-    uint64_t str[2] = {(uint64_t)a->ldc * es, sharded ? (uint64_t)a->c_shard_stride * es : (uint64_t)a->ldc * es * (uint64_t)a->M};
+    const bool by_shard = a->c_shard_stride > 0;
+    uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)(by_shard ? M_s : a->M), (uint64_t)(by_shard ? kp.m_shards : 1)};
+    uint64_t str[2] = {(uint64_t)a->ldc * es, by_shard ? (uint64_t)a->c_shard_stride * es : (uint64_t)a->ldc * es * (uint64_t)a->M};
     uint32_t box[3] = {(uint32_t)(f32 ? 32 : 64), (uint32_t)BM, 1};
     const void* out[3] = {a->c, a->c2, a->c3};
     CUtensorMap* map[3] = {&maps.C, &maps.S1, &maps.S2};
@@ -1143,8 +1157,9 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     kp.tma_epi = 2;
   if (a->c_shards != nullptr && a->epi == EPI_BF16_ACC && kp.tma_epi != 2)
     OB_FAIL(-18, "EPI_BF16_ACC towards c_shards needs the staged epilogue (16-byte aligned rows, local partial in c)");
-  return CG == 2 ? launch_layout<2>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream)
-                 : launch_layout<1>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
+  if (CG == 2) return launch_layout<2, BN_WIDE>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
+  if (BN == BN_NARROW) return launch_layout<1, BN_NARROW>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
+  return launch_layout<1, BN_WIDE>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
 }
 
 extern "C" const char* ob_last_error() { return ob::last_error_buf(); }

@@ -141,6 +141,34 @@ def test_gemm_weight_gradient_in_k_slices(K, M, N, Kd):
     _check_status()
 
 
+@pytest.mark.parametrize("M,N,Kd", [
+    (8, 8, 64), (128, 64, 72), (328, 1024, 200), (264, 136, 1000),
+    (1000, 1024, 1024), (1024, 1160, 320),   # 128 tiles of 128 x 64; 152: one more than fit at once, back to pairs
+])
+def test_gemm_small_problems_in_every_layout(K, M, N, Kd):
+    """Problems of one wave of 128 x 64 tiles, ragged in every extent: the three layouts, the fp32 epilogue, and the gated
+    one, which stays on the larger tiles."""
+    torch.manual_seed(31)
+    a = torch.randn(M, Kd, device="cuda", dtype=torch.bfloat16)
+    b, b2 = (torch.randn(N, Kd, device="cuda", dtype=torch.bfloat16) * Kd ** -0.5 for _ in range(2))
+    want = a.float() @ b.float().t()
+    c = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+    K.gemm(a, b, c, M, N, Kd)
+    assert rel_err(c, want) < 4e-3     # one bf16 rounding
+    cf = torch.zeros(M, N, device="cuda")
+    K.gemm(a, b, cf, M, N, Kd, epi=K.EPI_F32)
+    assert rel_err(cf, want) < 2e-5
+    c.zero_()
+    K.gemm(a, b.t().contiguous(), c, M, N, Kd, b_mn=True)
+    assert rel_err(c, want) < 4e-3
+    cf.zero_()
+    K.gemm(a.t().contiguous(), b.t().contiguous(), cf, M, N, Kd, a_mn=True, b_mn=True, epi=K.EPI_F32_ACC)
+    assert rel_err(cf, want) < 2e-5
+    K.gemm(a, b, c, M, N, Kd, epi=K.EPI_SWIGLU, b2=b2, ldb=Kd)
+    assert rel_err(c, ref.glu(want, a.float() @ b2.float().t(), "silu")) < 8e-3
+    _check_status()
+
+
 def test_gemm_sharded_operands(K):
     dev = "cuda"
     torch.manual_seed(1)
