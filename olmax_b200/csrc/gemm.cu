@@ -28,6 +28,9 @@
 // the A operand's row shards is fused in (`ag_on_a`: the copy warps pull the peers' rows while the tensor cores work
 // on the local rows), and the reduce-scatter of a row-parallel output is fused into the epilogue (row block s of
 // the partial product, plus an optional local partial sum, is stored into GPU s's staging slot).
+// Several weights that lie behind one another in memory and share an input (q / k / v, gate / up) are multiplied as one
+// matrix while their activations and gradients stay separate tensors: the output columns (forward), the contraction
+// (dgrad) or the output rows (wgrad) then run over up to three tensors, each with a tensor map of its own (`seg`).
 // Epilogues: bf16 store, fp32 store / accumulate / red.add, and the gated-MLP epilogue act(gate) * up computed from
 // a tile whose 256 accumulator columns are 128 gate columns followed by 128 up columns.
 //
@@ -35,6 +38,7 @@
 // `olmax/nn/mlp.py:69-73` (gated MLP).
 #include "gemm.h"
 
+#include <limits.h>
 #include <stdlib.h>
 
 #include "host_common.h"
@@ -64,6 +68,8 @@ struct Geo {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * EPI_STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
 };
 
+enum { SEG_NONE = 0, SEG_A_K = 1, SEG_A_M = 2, SEG_C_N = 3 };
+
 struct KernelParams {
   int M, N, Kc;
   int M_s, N_s, Kc_s;
@@ -81,6 +87,8 @@ struct KernelParams {
   int* status;
   int split, full_items, total_items;   // split-K tail: work items [full_items, total_items) are k slices of tiles
   int group_m;                 // tile rasterisation group (M tiles)
+  int seg;                     // SEG_*: which operand comes in segments
+  int seg_end[2];              // where segments 1 and 2 begin along the segmented extent (multiples of BM)
   int m_rot;                   // rotation of the M tile order (tiles), see decode_tile
   int a_single, b_single;      // MN-major operand fetched with one 4-D TMA box per stage instead of 64-wide boxes
   int tma_epi;                 // 1: outputs leave through shared memory + TMA store / reduce-add (tmC valid)
@@ -193,6 +201,20 @@ __device__ __forceinline__ void decode_work(const KernelParams& p, int w, int k_
     k_begin = (int)((long long)k_iters * sl / p.split);
     k_count = (int)((long long)k_iters * (sl + 1) / p.split) - k_begin;
   }
+}
+
+// The map of the segment that holds position `x` of the segmented extent; x becomes the position inside the segment.
+__device__ __forceinline__ const CUtensorMap* pick_segment(const CUtensorMap* s0, const CUtensorMap* s1, const CUtensorMap* s2,
+                                                           const KernelParams& p, int& x) {
+  if (x >= p.seg_end[1]) {
+    x -= p.seg_end[1];
+    return s2;
+  }
+  if (x >= p.seg_end[0]) {
+    x -= p.seg_end[0];
+    return s1;
+  }
+  return s0;
 }
 
 template <bool A_MN, bool B_MN, int CG, int BN>
@@ -313,6 +335,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             ag_ready_idx = ag_idx;
           }
         }
+        const CUtensorMap* mapA = &tmA;
+        int ka = k_glob, ma = m0;   // position in the A operand (segment)
+        if (p.seg == SEG_A_K) mapA = pick_segment(&tmA, &tmS1, &tmS2, p, ka);
+        if (p.seg == SEG_A_M) mapA = pick_segment(&tmA, &tmS1, &tmS2, p, ma);
         uint8_t* sa = smem + stage * STAGE_BYTES;
         uint8_t* sb = sa + A_STAGE_BYTES;
         if (leader && !dead) {
@@ -321,13 +347,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             if (A_MN) {
               if (p.a_single) {
                 // one 4-D box: (64 elements, 64 k-rows, 2 column blocks): lands as [block][k][128 B]
-                tma_load_4d(sa, &tmA, &full_bar[stage], 0, k_glob, m0 >> 6, 0);
+                tma_load_4d(sa, mapA, &full_bar[stage], 0, ka, ma >> 6, 0);
               } else {
-                tma_load_3d(sa, &tmA, &full_bar[stage], m0, k_glob, 0);
-                tma_load_3d(sa + MN_BLOCK_BYTES, &tmA, &full_bar[stage], m0 + 64, k_glob, 0);
+                tma_load_3d(sa, mapA, &full_bar[stage], ma, ka, 0);
+                tma_load_3d(sa + MN_BLOCK_BYTES, mapA, &full_bar[stage], ma + 64, ka, 0);
               }
             } else {
-              tma_load_3d(sa, &tmA, &full_bar[stage], k_glob, m0, 0);
+              tma_load_3d(sa, mapA, &full_bar[stage], ka, ma, 0);
             }
             if (B_MN) {
               // dims (N, Kc_s, k_shards): BN / 64 64-wide blocks along N
@@ -351,13 +377,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
             if (A_MN) {
               if (p.a_single) {
-                tma_load_4d_pair(sa, &tmA, fb, 0, k_glob, m0 >> 6, 0);
+                tma_load_4d_pair(sa, mapA, fb, 0, ka, ma >> 6, 0);
               } else {
-                tma_load_3d_pair(sa, &tmA, fb, m0, k_glob, 0);
-                tma_load_3d_pair(sa + MN_BLOCK_BYTES, &tmA, fb, m0 + 64, k_glob, 0);
+                tma_load_3d_pair(sa, mapA, fb, ma, ka, 0);
+                tma_load_3d_pair(sa + MN_BLOCK_BYTES, mapA, fb, ma + 64, ka, 0);
               }
             } else {
-              tma_load_3d_pair(sa, &tmA, fb, k_glob, m0, 0);
+              tma_load_3d_pair(sa, mapA, fb, ka, ma, 0);
             }
             if (B_MN) {
               const int n0 = n_local0 + cta_rank * BNL;   // this CTA's half of the tile's columns: two 64-wide blocks
@@ -633,7 +659,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             if (store_thread) {
               if (m_valid > 0) {   // a pair tile's second half may lie wholly below the shard
                 if (p.epi == EPI_F32_ACC) tma_reduce_add_3d(&tmC, stage_buf, n_glob0 + c0, out_row, out_z);
-                else tma_store_3d(&tmC, stage_buf, n_glob0 + c0, out_row, out_z);
+                else {
+                  int n = n_glob0 + c0;
+                  const CUtensorMap* mapC = p.seg == SEG_C_N ? pick_segment(&tmC, &tmS1, &tmS2, p, n) : &tmC;
+                  tma_store_3d(mapC, stage_buf, n, out_row, out_z);
+                }
               }
               tma_store_commit();
             }
@@ -845,7 +875,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 
 constexpr int MAX_DEVICES = 64;
 
-// The tensor maps of a launch; S1 / S2 are the second and third output of the gated epilogue.
+// The tensor maps of a launch; S1 / S2 are the second and third output of the gated epilogue, or the segments after the
+// first of a segmented operand.
 struct Maps {
   CUtensorMap A, B, B2, C, S1, S2;
 };
@@ -1003,32 +1034,58 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     kp.pf_dst_stride = a->pf_dst_stride; kp.pf_off = a->pf_off; kp.pf_bytes = a->pf_bytes;
   }
 
+  // Segments: up to three tensors side by side along one extent, each boundary on a tile boundary (BM).
+  const int* seg_len = a->seg_len;
+  const int n_seg = a->seg == SEG_NONE ? 1 : (seg_len[2] > 0 ? 3 : 2);
+  kp.seg = a->seg;
+  kp.seg_end[0] = kp.seg_end[1] = INT_MAX;
+  if (a->seg != SEG_NONE) {
+    if (a->seg < SEG_NONE || a->seg > SEG_C_N) OB_FAIL(-19, "unknown segmented operand %d", a->seg);
+    const int extent = a->seg == SEG_A_K ? a->Kc : a->seg == SEG_A_M ? a->M : a->N;
+    if (seg_len[0] <= 0 || seg_len[1] <= 0 || seg_len[2] < 0 ||
+        (long long)seg_len[0] + seg_len[1] + seg_len[2] != extent)
+      OB_FAIL(-19, "segments %d + %d + %d do not add up to %d", seg_len[0], seg_len[1], seg_len[2], extent);
+    if (seg_len[0] % BM || seg_len[1] % BM || seg_len[2] % BM) OB_FAIL(-19, "segments must be multiples of %d", BM);
+    if (a->seg_ptr[0] == nullptr || (n_seg == 3 && a->seg_ptr[1] == nullptr)) OB_FAIL(-19, "segment without a tensor");
+    if (kp.m_shards * kp.n_shards * kp.k_shards != 1 || a->ag_src != nullptr || a->c_shards != nullptr || glu ||
+        (a->seg == SEG_A_K && a->a_mn) || (a->seg == SEG_A_M && !a->a_mn) || (a->seg == SEG_C_N && a->epi != EPI_BF16))
+      OB_FAIL(-19, "segments go with unsharded GEMMs: K-major A along K, MN-major A along M, or a bf16 output along N");
+    kp.seg_end[0] = seg_len[0];
+    if (n_seg == 3) kp.seg_end[1] = seg_len[0] + seg_len[1];
+  }
+
   Maps maps;
   memset(&maps, 0, sizeof(maps));
-  CUtensorMap &tA = maps.A, &tB = maps.B, &tB2 = maps.B2;
+  CUtensorMap &tB = maps.B, &tB2 = maps.B2;
   int rc;
   kp.a_single = kp.b_single = 0;
-  // (every tile must start on a multiple of 64 along M: with row shards of M_s rows, tile starts are s * M_s + 128 t)
-  if (a->a_mn && a->M % 64 == 0 && M_s % 64 == 0 && !a->multi_box_mn) {
-    // view [Kc, M] as (64, Kc, M/64): a tile is ONE box of 64 x 64 x 2, which lands in shared memory as two
-    // [64 k][128 B] blocks, the MN-major layout the MMA descriptor expects
-    uint64_t dims[4] = {64, (uint64_t)a->Kc, (uint64_t)a->M / 64, 1};
-    uint64_t str[3] = {(uint64_t)a->lda * 2, 128, (uint64_t)a->lda * 2 * (uint64_t)a->Kc};
-    uint32_t box[4] = {64, (uint32_t)BK, 2, 1};
-    rc = encode_tmap(&tA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    kp.a_single = 1;
-  } else if (a->a_mn) {  // stored [Kc, M], M contiguous
-    uint64_t dims[3] = {(uint64_t)a->M, (uint64_t)a->Kc, 1};
-    uint64_t str[2] = {(uint64_t)a->lda * 2, (uint64_t)a->lda * 2 * (uint64_t)a->Kc};
-    uint32_t box[3] = {64, (uint32_t)BK, 1};
-    rc = encode_tmap(&tA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
-  } else {  // stored [M, Kc], Kc contiguous
-    uint64_t dims[3] = {(uint64_t)a->Kc, (uint64_t)a->M, 1};
-    uint64_t str[2] = {(uint64_t)a->lda * 2, (uint64_t)a->lda * 2 * (uint64_t)a->M};
-    uint32_t box[3] = {(uint32_t)BK, (uint32_t)BM, 1};
-    rc = encode_tmap(&tA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+  for (int g = 0; g < (a->seg == SEG_C_N ? 1 : n_seg); ++g) {
+    CUtensorMap* map = g == 0 ? &maps.A : g == 1 ? &maps.S1 : &maps.S2;
+    const void* ptr = g == 0 ? a->a : a->seg_ptr[g - 1];
+    const long long lda = g == 0 ? a->lda : a->seg_ld[g - 1];
+    const int M = a->seg == SEG_A_M ? seg_len[g] : a->M, Kc = a->seg == SEG_A_K ? seg_len[g] : a->Kc;
+    // (every tile must start on a multiple of 64 along M: with row shards of M_s rows, tile starts are s * M_s + 128 t)
+    if (a->a_mn && a->M % 64 == 0 && M_s % 64 == 0 && !a->multi_box_mn) {
+      // view [Kc, M] as (64, Kc, M/64): a tile is ONE box of 64 x 64 x 2, which lands in shared memory as two
+      // [64 k][128 B] blocks, the MN-major layout the MMA descriptor expects
+      uint64_t dims[4] = {64, (uint64_t)Kc, (uint64_t)M / 64, 1};
+      uint64_t str[3] = {(uint64_t)lda * 2, 128, (uint64_t)lda * 2 * (uint64_t)Kc};
+      uint32_t box[4] = {64, (uint32_t)BK, 2, 1};
+      rc = encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, ptr, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+      kp.a_single = 1;
+    } else if (a->a_mn) {  // stored [Kc, M], M contiguous
+      uint64_t dims[3] = {(uint64_t)M, (uint64_t)Kc, 1};
+      uint64_t str[2] = {(uint64_t)lda * 2, (uint64_t)lda * 2 * (uint64_t)Kc};
+      uint32_t box[3] = {64, (uint32_t)BK, 1};
+      rc = encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    } else {  // stored [M, Kc], Kc contiguous
+      uint64_t dims[3] = {(uint64_t)Kc, (uint64_t)M, 1};
+      uint64_t str[2] = {(uint64_t)lda * 2, (uint64_t)lda * 2 * (uint64_t)M};
+      uint32_t box[3] = {(uint32_t)BK, (uint32_t)BM, 1};
+      rc = encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    }
+    if (rc) return rc;
   }
-  if (rc) return rc;
   const long long bss = a->b_shard_stride > 0 ? a->b_shard_stride : 0;
   if (a->b_mn && a->N % 64 == 0 && !a->multi_box_mn) {
     uint64_t sstride = kp.k_shards > 1 ? (uint64_t)bss * 2 : (uint64_t)a->ldb * 2 * (uint64_t)Kc_s;
@@ -1131,21 +1188,30 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     const bool f32 = a->epi == EPI_F32 || a->epi == EPI_F32_ACC;
     const uint64_t es = f32 ? 4 : 2;
     const bool by_shard = a->c_shard_stride > 0;
-    uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)(by_shard ? M_s : a->M), (uint64_t)(by_shard ? kp.m_shards : 1)};
-    uint64_t str[2] = {(uint64_t)a->ldc * es, by_shard ? (uint64_t)a->c_shard_stride * es : (uint64_t)a->ldc * es * (uint64_t)a->M};
-    uint32_t box[3] = {(uint32_t)(f32 ? 32 : 64), (uint32_t)BM, 1};
+    const int n_out = glu && a->c2 != nullptr ? 3 : a->seg == SEG_C_N ? n_seg : 1;
     const void* out[3] = {a->c, a->c2, a->c3};
+    long long ldc[3] = {a->ldc, a->ldc, a->ldc};
+    if (a->seg == SEG_C_N) {
+      out[1] = a->seg_ptr[0]; out[2] = a->seg_ptr[1];
+      ldc[1] = a->seg_ld[0]; ldc[2] = a->seg_ld[1];
+    }
+    uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)(by_shard ? M_s : a->M), (uint64_t)(by_shard ? kp.m_shards : 1)};
+    uint32_t box[3] = {(uint32_t)(f32 ? 32 : 64), (uint32_t)BM, 1};
     CUtensorMap* map[3] = {&maps.C, &maps.S1, &maps.S2};
-    const int n_out = glu && a->c2 != nullptr ? 3 : 1;
-    bool aligned = str[0] % 16 == 0 && str[1] % 16 == 0;
-    for (int i = 0; i < n_out; ++i) aligned = aligned && (reinterpret_cast<uintptr_t>(out[i]) & 15) == 0;
+    bool aligned = true;
+    for (int i = 0; i < n_out; ++i)
+      aligned = aligned && (reinterpret_cast<uintptr_t>(out[i]) & 15) == 0 && (uint64_t)ldc[i] * es % 16 == 0 &&
+                (!by_shard || (uint64_t)a->c_shard_stride * es % 16 == 0);
     for (int i = 0; i < n_out && aligned; ++i) {
+      uint64_t str[2] = {(uint64_t)ldc[i] * es, by_shard ? (uint64_t)a->c_shard_stride * es : (uint64_t)ldc[i] * es * (uint64_t)a->M};
+      if (a->seg == SEG_C_N) dims[0] = (uint64_t)seg_len[i];
       rc = encode_tmap(map[i], f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, out[i], dims, str, box,
                        CU_TENSOR_MAP_SWIZZLE_128B);
       if (rc) return rc;
     }
     kp.tma_epi = aligned ? 1 : 0;
   }
+  if (a->seg == SEG_C_N && kp.tma_epi != 1) OB_FAIL(-19, "a segmented output needs 16-byte aligned rows");
   if (kp.split > 1 && a->epi == EPI_F32_ACC && kp.tma_epi != 1) {   // no atomic path for the slices: whole tiles only
     kp.split = 1;
     kp.full_items = kp.total_items = total;

@@ -71,6 +71,14 @@ typedef struct ObGemmArgs {
   int ag_on_a;
   // 1: never cut the tiles of the last partial wave into k slices (accumulating fp32 epilogues do by default)
   int no_split_k;
+  // Segments (0: none): one extent runs over up to three tensors side by side, so that weights which lie behind one
+  // another in memory are multiplied as one matrix.  seg = 1: the contraction of a K-major A (a, seg_ptr[0], seg_ptr[1]
+  // are [M, seg_len[i]]); 2: the rows of an MN-major A ([Kc, seg_len[i]]); 3: the columns of a bf16 output (c,
+  // seg_ptr[i] are [M, seg_len[i]]).  Lengths are multiples of 128 and add up to the extent; seg_len[2] = 0: two.
+  int seg;
+  int seg_len[3];
+  const void* seg_ptr[2];
+  long long seg_ld[2];
 } ObGemmArgs;
 
 int ob_gemm_bf16(const ObGemmArgs* args, cudaStream_t stream);

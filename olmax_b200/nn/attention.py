@@ -20,7 +20,7 @@ from ..parallel import collectives as coll
 from ..parallel.context import CPStrategy, context_parallel_attention
 from ..parallel.mesh import TPStyle
 from ..types import StrEnum
-from .linear import Linear
+from .linear import Linear, linear_group
 from .module import Module, current_build_context
 from .normalization import NormalizerConfig, RMSNorm, RMSNormConfig
 from .rope import BufferCache, RotaryPositionalEmbedding, RotaryPositionalEmbeddingConfig
@@ -127,9 +127,7 @@ class MultiheadSelfAttention(Module):
             q, k, v = F.tp_column_linears(x, tpc, (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight))
         else:
             x = coll.seq_all_gather(x, tp)
-            q = self.q_proj(x)
-            k = self.k_proj(x)
-            v = self.v_proj(x)
+            q, k, v = linear_group((self.q_proj, self.k_proj, self.v_proj), x)
         T = q.shape[0]
         S = T // batch_size
         heads_q = self.local_heads if self.use_head_qk_norm else 1

@@ -11,7 +11,7 @@ from ..parallel import collectives as coll
 from ..parallel.mesh import TPStyle
 from .module import Module
 
-__all__ = ["Linear"]
+__all__ = ["Linear", "linear_group"]
 
 
 class Linear(Module):
@@ -39,3 +39,16 @@ class Linear(Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         return F.linear(x, self.weight, self.bias)
+
+
+def linear_group(mods, x: torch.Tensor):
+    """``m(x)`` for every module of a group that reads one input, as one GEMM where they are plain unhooked
+    :class:`Linear` layers whose weights can be joined."""
+    if all(type(m) is Linear and "forward" not in m.__dict__ and not _hooked(m) for m in mods):
+        return F.linears(x, [m.weight for m in mods], [m.bias for m in mods])
+    return tuple(m(x) for m in mods)
+
+
+def _hooked(m: torch.nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or torch.nn.modules.module._has_any_global_hook())

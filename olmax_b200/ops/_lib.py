@@ -71,6 +71,10 @@ class ObGemmArgs(ctypes.Structure):
         ("no_tma_epilogue", ctypes.c_int),
         ("ag_on_a", ctypes.c_int),
         ("no_split_k", ctypes.c_int),
+        ("seg", ctypes.c_int),
+        ("seg_len", ctypes.c_int * 3),
+        ("seg_ptr", ctypes.c_void_p * 2),
+        ("seg_ld", ctypes.c_longlong * 2),
     ]
 
 

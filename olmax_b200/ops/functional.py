@@ -23,7 +23,7 @@ from ..parallel import collectives as coll
 from . import reference as ref
 
 __all__ = [
-    "linear", "gated_mlp", "rms_norm", "layer_norm", "rope", "attention", "attention_block_fwd", "attention_block_bwd",
+    "linear", "linears", "gated_mlp", "rms_norm", "layer_norm", "rope", "attention", "attention_block_fwd", "attention_block_bwd",
     "embedding", "linear_cross_entropy", "glu", "tp_column_linears", "tp_row_linear",
 ]
 
@@ -125,6 +125,49 @@ def _gemm_wgrad(dy2: torch.Tensor, x2: torch.Tensor, handle) -> None:
         K.gemm(dy2, x2, dst, N, Kd, M, a_mn=True, b_mn=True, epi=K.EPI_F32_ACC, alpha=scale, ldc=Kd, prefetch=pf, **kw)
 
 
+def _joined(handles) -> bool:
+    """Whether two or three weights can be multiplied as one matrix: unsharded, with the same input width, behind one
+    another in the flat buffers (which they are when registered in a row), rows in whole GEMM tiles of 128."""
+    first = handles[0]
+    if not 2 <= len(handles) <= 3 or first.shard_count != 1:
+        return False
+    end, width = first.meta.offset, first.meta.local_shape[-1]
+    for h in handles:
+        m = h.meta
+        if (h.store is not first.store or h.unit is not first.unit or len(m.local_shape) != 2 or m.offset != end
+                or m.local_shape[1] != width or m.local_shape[0] % 128):
+            return False
+        end = m.offset + m.numel_local
+    return True
+
+
+def _joined_fwd(x2: torch.Tensor, handles) -> list:
+    """[x2 @ W_i^T] of joined weights, one GEMM."""
+    M, Kd = x2.shape
+    ys = [torch.empty((M, h.tp_shape[0]), dtype=torch.bfloat16, device=x2.device) for h in handles]
+    first, _ = handles[0].pieces()
+    K.gemm(x2, first, ys[0], M, sum(y.shape[1] for y in ys), Kd, ldb=Kd, seg=K.SEG_C_N, seg_rest=ys[1:])
+    return ys
+
+
+def _joined_dgrad(dys, handles) -> torch.Tensor:
+    """sum_i dy_i @ W_i of joined weights, one GEMM (the sum is formed in its fp32 accumulators)."""
+    M = dys[0].shape[0]
+    Kd = handles[0].tp_shape[1]
+    first, _ = handles[0].pieces()
+    dx = torch.empty((M, Kd), dtype=torch.bfloat16, device=dys[0].device)
+    K.gemm(dys[0], first, dx, M, Kd, sum(dy.shape[1] for dy in dys), b_mn=True, ldb=Kd, seg=K.SEG_A_K, seg_rest=dys[1:])
+    return dx
+
+
+def _joined_wgrad(dys, x2: torch.Tensor, handles) -> None:
+    """dW_i += scale * dy_i^T @ x2 of joined weights, one GEMM into their neighbouring accumulators."""
+    M, Kd = x2.shape
+    dst, _, scale = handles[0].grad_pieces()
+    K.gemm(dys[0], x2, dst, sum(dy.shape[1] for dy in dys), Kd, M, a_mn=True, b_mn=True, epi=K.EPI_F32_ACC, alpha=scale,
+           ldc=Kd, seg=K.SEG_A_M, seg_rest=dys[1:])
+
+
 # ----------------------------------------------------------------------------------------------------------------------
 # Linear
 # ----------------------------------------------------------------------------------------------------------------------
@@ -169,6 +212,33 @@ class _LinearFn(torch.autograd.Function):
 def linear(x: torch.Tensor, handle, bias_handle=None) -> torch.Tensor:
     """``x @ W^T (+ b)`` with W ``(out, in)`` (``olmax/nn/functional.py:14-27``)."""
     return _LinearFn.apply(x, handle, bias_handle)
+
+
+class _JoinedLinearsFn(torch.autograd.Function):
+    """(x @ W_i^T for every weight i) of joined weights (:func:`_joined`): one GEMM forward, one for the input gradient
+    (which would otherwise be a sum of one bf16 tensor per weight) and one for the weight gradients."""
+
+    @staticmethod
+    def forward(ctx, x, *handles):
+        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        ctx.handles, ctx.shape = handles, x.shape
+        ctx.save_for_backward(x2)
+        return tuple(y.view(*x.shape[:-1], y.shape[-1]) for y in _joined_fwd(x2, handles))
+
+    @staticmethod
+    def backward(ctx, *dys):
+        (x2,) = ctx.saved_tensors
+        dys = [dy.reshape(-1, dy.shape[-1]).contiguous() for dy in dys]
+        dx = _joined_dgrad(dys, ctx.handles).view(ctx.shape) if ctx.needs_input_grad[0] else None
+        _joined_wgrad(dys, x2, ctx.handles)
+        return (dx,) + (None,) * len(ctx.handles)
+
+
+def linears(x: torch.Tensor, handles, bias_handles):
+    """``linear(x, h, b)`` for every weight of a group that shares its input, as one GEMM where they can be joined."""
+    if all(b is None for b in bias_handles) and _on_gpu(x) and _joined(handles):
+        return _JoinedLinearsFn.apply(x, *handles)
+    return tuple(linear(x, h, b) for h, b in zip(handles, bias_handles))
 
 
 # ----------------------------------------------------------------------------------------------------------------------
@@ -262,9 +332,14 @@ class _GatedMLPFn(torch.autograd.Function):
             del da
             _gemm_wgrad(dy2, a, down)
             del a
+            dx = None
+            if tpc is None and _joined((gate, up)):
+                _joined_wgrad((dg, du), x2, (gate, up))
+                if ctx.needs_input_grad[0]:
+                    dx = _joined_dgrad((dg, du), (gate, up))
+                return (dx.view(ctx.shape) if dx is not None else None), None, None, None, None, None, None
             _gemm_wgrad(dg, x2, gate)
             _gemm_wgrad(du, x2, up)
-            dx = None
             if ctx.needs_input_grad[0]:
                 dx = _gemm_dgrad(dg, gate)
                 if tpc is not None:

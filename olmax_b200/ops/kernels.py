@@ -23,6 +23,7 @@ from ._lib import KernelError, ObAttnArgs, ObGemmArgs, check, lib, register_sign
 
 __all__ = [
     "EPI_BF16", "EPI_F32", "EPI_F32_ACC", "EPI_F32_RED", "EPI_SWIGLU", "EPI_GEGLU", "EPI_BF16_ACC",
+    "SEG_NONE", "SEG_A_K", "SEG_A_M", "SEG_C_N",
     "gemm", "flash_attn_fwd", "flash_attn_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rmsnorm_rope_fwd", "rmsnorm_rope_bwd", "rope", "glu_fwd", "glu_bwd",
     "embed_gather", "embed_scatter", "ce_fwd_bwd", "ce_vp_stats", "ce_vp_grad", "count_valid", "adamw", "sumsq", "clip_coef", "cast_f32_bf16",
     "layernorm_fwd", "layernorm_bwd", "gather_shards", "scatter_add_shards", "allreduce_p2p", "allreduce_multimem",
@@ -32,6 +33,7 @@ __all__ = [
 ]
 
 EPI_BF16, EPI_F32, EPI_F32_ACC, EPI_F32_RED, EPI_SWIGLU, EPI_GEGLU, EPI_BF16_ACC = range(7)
+SEG_NONE, SEG_A_K, SEG_A_M, SEG_C_N = range(4)
 
 _LAUNCHES = 0
 
@@ -139,8 +141,11 @@ def gemm(
     m_shard_rot: int = 0,
     ag_on_a: bool = False,
     no_split_k: bool = False,
+    seg: int = SEG_NONE,
+    seg_rest: Sequence[torch.Tensor] = (),
 ) -> None:
-    """``C[M, N] (+)= alpha * A[M, K] . B[K, N]``; see ``csrc/gemm.h`` for operand layouts and sharding."""
+    """``C[M, N] (+)= alpha * A[M, K] . B[K, N]``; see ``csrc/gemm.h`` for operand layouts and sharding.  ``seg``: the
+    operand it names (``a``, or ``c``) goes on in the tensors ``seg_rest``, one or two more beside the first."""
     _req_bf16(a, b, b2)
     args = ObGemmArgs()
     args.a = a.data_ptr()
@@ -170,6 +175,16 @@ def gemm(
     args.multi_box_mn = int(multi_box_mn)
     args.ag_on_a = int(ag_on_a)
     args.no_split_k = int(no_split_k)
+    if seg != SEG_NONE:
+        pieces = (c if seg == SEG_C_N else a, *seg_rest)
+        if not 2 <= len(pieces) <= 3 or any(t.stride(-1) != 1 for t in pieces):
+            raise KernelError("a segmented GEMM operand has two or three pieces with contiguous rows")
+        _req_bf16(*pieces)
+        args.seg = seg
+        for i, t in enumerate(pieces):
+            args.seg_len[i] = t.shape[-1]
+            if i > 0:
+                args.seg_ptr[i - 1], args.seg_ld[i - 1] = t.data_ptr(), t.stride(0)
     if prefetch is not None:
         table, dst_ptr, dst_stride, off, nbytes, shards, rank = prefetch
         args.pf_src, args.pf_dst, args.pf_dst_stride = table.data_ptr(), dst_ptr, dst_stride

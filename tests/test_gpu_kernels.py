@@ -169,6 +169,33 @@ def test_gemm_small_problems_in_every_layout(K, M, N, Kd):
     _check_status()
 
 
+@pytest.mark.parametrize("M,Kd,widths", [
+    (8, 64, (128, 128)), (1000, 1024, (1024, 128, 128)), (520, 136, (384, 256, 128)), (2056, 512, (1408, 1408)),
+])
+def test_gemm_segmented_operands(K, M, Kd, widths):
+    """Weights behind one another as one matrix: the outputs, input gradient and weight gradients of the separate GEMMs."""
+    torch.manual_seed(37)
+    N = sum(widths)
+    x = torch.randn(M, Kd, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(N, Kd, device="cuda", dtype=torch.bfloat16) * Kd ** -0.5
+    ys = [torch.zeros(M, n, device="cuda", dtype=torch.bfloat16) for n in widths]
+    K.gemm(x, w, ys[0], M, N, Kd, seg=K.SEG_C_N, seg_rest=ys[1:])
+    for y, wi in zip(ys, w.split(widths)):
+        assert rel_err(y, x.float() @ wi.float().t()) < 4e-3
+    # gradients that are column slices of wider tensors keep their row strides
+    dys = [torch.randn(M, n + 8, device="cuda", dtype=torch.bfloat16)[:, :n] for n in widths]
+    dcat = torch.cat([d.float() for d in dys], 1)
+    dx = torch.zeros(M, Kd, device="cuda", dtype=torch.bfloat16)
+    K.gemm(dys[0], w, dx, M, Kd, N, b_mn=True, ldb=Kd, seg=K.SEG_A_K, seg_rest=dys[1:])
+    assert rel_err(dx, dcat @ w.float()) < 4e-3
+    dw = torch.zeros(N, Kd, device="cuda")
+    K.gemm(dys[0], x, dw, N, Kd, M, a_mn=True, b_mn=True, epi=K.EPI_F32_ACC, alpha=0.5, seg=K.SEG_A_M, seg_rest=dys[1:])
+    assert rel_err(dw, 0.5 * dcat.t() @ x.float()) < 2e-5
+    with pytest.raises(Exception):   # a boundary inside a tile
+        K.gemm(x, w[:192], ys[0][:, :64], M, 192, Kd, seg=K.SEG_C_N, seg_rest=[ys[1]])
+    _check_status()
+
+
 def test_gemm_sharded_operands(K):
     dev = "cuda"
     torch.manual_seed(1)
