@@ -733,6 +733,45 @@ def test_vocab_parallel_cross_entropy_kernels(K, softcap, z):
     _check_status()
 
 
+@pytest.mark.parametrize("rows,V,softcap", [
+    (3, 8, 0.0), (5, 1004, 0.0), (4, 8189, 20.0),   # shorter than a thread's batch; vectors of 4 but not of 8; scalar tails
+    (3, 12288, 0.0), (3, 12290, 0.0), (3, 12296, 30.0),   # exactly, and just beyond, what shared memory keeps of a row
+    (2, 50304, 0.0), (150 * 4, 20000, 0.0),          # several backward steps; more rows than blocks at once
+])
+def test_cross_entropy_row_lengths(K, rows, V, softcap):
+    """Loss, log-sum-exp and gradient against fp64; a row that starts with 4096 classes masked to -inf keeps its finite loss.
+    Tolerances: fp32 sums of V terms for the loss, one bf16 rounding (2^-9) for the gradient; with the soft-cap the
+    hardware tanh (2^-11 relative) enters both."""
+    torch.manual_seed(V)
+    ld = (V + 7) // 8 * 8
+    logits = (torch.randn(rows, ld, device="cuda") * 3)[:, :V]
+    if V >= 12288 and not softcap:
+        logits[0, :4096] = float("-inf")
+    labels = torch.randint(V - V // 2, V, (rows,), device="cuda")
+    labels[1] = -100
+    z = logits.double()
+    z = softcap * torch.tanh(z / softcap) if softcap else z
+    lse = torch.logsumexp(z, -1)
+    valid = labels != -100
+    want = (lse - z.gather(1, labels.clamp(min=0)[:, None])[:, 0])[valid].sum()
+    g = torch.softmax(z, -1)
+    g.scatter_add_(1, labels.clamp(min=0)[:, None], -torch.ones(rows, 1, device="cuda", dtype=torch.float64))
+    if softcap:
+        g *= 1 - torch.tanh(logits.double() / softcap) ** 2
+    g[~valid] = 0
+    stats, inv = torch.zeros(2, device="cuda"), torch.ones(1, device="cuda")
+    dl = torch.full((rows, ld), 5.0, device="cuda", dtype=torch.bfloat16)[:, :V]
+    lse_out = torch.empty(rows, device="cuda")
+    K.ce_fwd_bwd(logits, labels, dl, stats, inv, V=V, softcap=softcap, lse=lse_out)
+    assert (lse_out.double() - lse).abs().max().item() < (2e-2 if softcap else 2e-5)
+    assert abs(stats[0].item() - want.item()) < (1e-3 if softcap else 1e-5) * abs(want.item()) + 1e-5
+    assert rel_err(dl, g) < (1e-2 if softcap else 4e-3)
+    stats2 = torch.zeros(2, device="cuda")
+    K.ce_fwd_bwd(logits, labels, None, stats2, inv, V=V, softcap=softcap)
+    assert abs((stats2[0] - stats[0]).item()) < 1e-5 * abs(want.item()) + 1e-5
+    _check_status()
+
+
 def test_adamw_and_norm_kernels(K):
     dev = "cuda"
     torch.manual_seed(8)
