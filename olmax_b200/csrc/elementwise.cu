@@ -46,7 +46,7 @@ __device__ __forceinline__ void load8f(const float* p, float (&f)[8]) {
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
-// Sum over the TPR threads that share a row (TPR = 16 or 32: shuffles; TPR = 256: shuffles + shared memory).
+// Sum over the TPR threads that share a row (TPR = 16 or 32: shuffles; more: shuffles + shared memory).
 template <int TPR>
 __device__ __forceinline__ float row_sum(float v, float* red) {
   if (TPR <= 32) {
@@ -62,13 +62,13 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
     __syncthreads();
     float t = 0.f;
 #pragma unroll
-    for (int i = 0; i < TPR / 32; ++i) t += red[i];
+    for (int i = 0; i < TPR / 32; ++i) t += red[threadIdx.x / TPR * (TPR / 32) + i];
     return t;
   }
 }
 
 constexpr int NORM_THREADS = 256;
-constexpr int MAX_VPT = 4;  // most 8-element vectors per thread kept in registers (kernels are instantiated for 1, 2, 4)
+constexpr int MAX_VPT = 4;  // most 8-element vectors per thread kept in registers (kernels are instantiated for 1 to 4)
 
 // Rows are addressed as  base + (row / heads) * ld + (row % heads) * d   (heads = 1, ld = d: plain 2-D tensor).
 __device__ __forceinline__ long long row_offset(long long row, int heads, long long ld, int d) {
@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
     }
   }
   if (dw == nullptr) return;
-  // combine the row groups of this block in shared memory, then one atomic per element per block
+  // Combine the row groups of this block in shared memory, then one atomic per element per block.  Element vi * 8 + j sits
+  // at j * nvec + vi, so that the lanes of a warp (consecutive vi) hit different banks.
   for (int i = threadIdx.x; i < d; i += NORM_THREADS) dw_part[i] = 0.f;
   __syncthreads();
 #pragma unroll
@@ -245,13 +246,13 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
     if (vi < nvec) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        if (ROWS_PER_BLOCK > 1) atomicAdd(&dw_part[vi * 8 + j], dwacc[i][j]);
-        else dw_part[vi * 8 + j] = dwacc[i][j];
+        if (ROWS_PER_BLOCK > 1) atomicAdd(&dw_part[j * nvec + vi], dwacc[i][j]);
+        else dw_part[j * nvec + vi] = dwacc[i][j];
       }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < d; i += NORM_THREADS) atomicAdd(dw + i, dw_part[i] * dw_scale);
+  for (int i = threadIdx.x; i < d; i += NORM_THREADS) atomicAdd(dw + i, dw_part[(i & 7) * nvec + (i >> 3)] * dw_scale);
 }
 
 // LayerNorm (`olmax/nn/functional.py:30-49`): y = (x - mean) * rstd * w (+ b), statistics over the row in fp32 (the
@@ -780,6 +781,9 @@ static inline int resident_grid(Kernel kernel, long long work_blocks, size_t sme
 // Thread layout of the normalisation kernels for a row of d elements: TPR threads share a row and each keeps VPT
 // 8-element vectors of it in registers.  Instantiating the smallest VPT that covers d keeps the register count (and
 // with it the number of resident blocks, i.e. the bytes in flight) right for the common widths.
+// d = 1024 with 256 threads left half of them without a vector, and 4608 / 5120 with four vectors per thread left 40 %:
+// [65536, 1024] pre-norm forward 104 -> 95 us, backward 152 -> 123 us (128 threads per row); [5560, 5120] backward 76 -> 68 us
+// (three vectors); [1024, 512] backward 17 -> 12 us (a warp per row, and partial sums that do not collide in a bank).
 template <int T, int V>
 struct NormShape {
   static constexpr int TPR = T, VPT = V;
@@ -788,9 +792,11 @@ template <typename F>
 static inline int norm_dispatch(int d, const char* what, F&& launch) {
   if (d % 8 != 0) OB_FAIL(-1, "%s: d (%d) must be a multiple of 8", what, d);
   if (d <= 128) launch(NormShape<16, 1>{});
-  else if (d <= 512) launch(NormShape<16, 4>{});
+  else if (d <= 512) launch(NormShape<32, 2>{});
+  else if (d <= 1024) launch(NormShape<128, 1>{});
   else if (d <= 2048) launch(NormShape<NORM_THREADS, 1>{});
   else if (d <= 4096) launch(NormShape<NORM_THREADS, 2>{});
+  else if (d <= 6144) launch(NormShape<NORM_THREADS, 3>{});
   else if (d <= NORM_THREADS * 8 * MAX_VPT) launch(NormShape<NORM_THREADS, 4>{});
   else OB_FAIL(-2, "%s: d (%d) too large (max %d)", what, d, NORM_THREADS * 8 * MAX_VPT);
   OB_CUDA_OK(cudaGetLastError());

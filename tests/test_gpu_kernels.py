@@ -492,6 +492,28 @@ def test_blockwise_attention_composes_to_full_attention(K):
     _check_status()
 
 
+@pytest.mark.parametrize("rows", [1, 7, 2049])
+@pytest.mark.parametrize("d", [256, 520, 768, 1024, 1032, 4104, 4608, 6144, 6152])
+def test_rmsnorm_thread_layouts(K, rows, d):
+    """Row lengths at the edges of the thread layouts (two rows per block up to 1024, three vectors per thread up to 6144):
+    pre-norm forward and its backward with the residual gradient.  One bf16 rounding per output (2^-9); dw in fp32."""
+    torch.manual_seed(d)
+    x, res, dy, ds = (torch.randn(rows, d, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    w = (torch.randn(d, device="cuda") * 0.1 + 1).to(torch.bfloat16)
+    y, h, dx = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+    rstd, dw = torch.empty(rows, device="cuda"), torch.ones(d, device="cuda")
+    K.rmsnorm_fwd(x, w, y, rows=rows, d=d, eps=1e-5, res=res, sum_out=h, rstd=rstd, add_before=True)
+    hf = (x.float() + res.float()).to(torch.bfloat16).float().requires_grad_(True)
+    wf = w.float().requires_grad_(True)
+    yr = ref.rms_norm(hf, wf, 1e-5)
+    gh, gw = torch.autograd.grad(yr, (hf, wf), dy.float())
+    assert rel_err(h, hf.detach()) < 1e-6 and rel_err(y, yr) < 4e-3
+    K.rmsnorm_bwd(dy, h, w, rstd, dx, rows=rows, d=d, dw=dw, dsum=ds, dw_scale=0.5)
+    assert rel_err(dx, gh + ds.float()) < 4e-3
+    assert rel_err(dw, 1 + 0.5 * gw) < 1e-5
+    _check_status()
+
+
 @pytest.mark.parametrize("rows,d,bias", [(300, 512, True), (70, 4096, True), (33, 8192, False), (257, 128, True),
                                            (65, 2048, True)])
 def test_layernorm(K, rows, d, bias):
