@@ -8,6 +8,8 @@
 // (`olmax/optim/config.py:125-156`, `olmax/optim/utils.py:15-38`).
 #include "optim_loss.h"
 #include "host_common.h"
+
+#include <limits.h>
 #include "sm100.cuh"
 
 namespace ob {
@@ -300,36 +302,54 @@ __global__ void count_valid_kernel(const long long* __restrict__ labels, long lo
 }
 
 // p, m, v, g: fp32 [n]; shadow: bf16 [n] (optional).  g_eff = g * (*gscale) (gscale optional, device scalar).
-__global__ void adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float* __restrict__ g,
+// One block per span of 2 x 256 vectors, in launch order: 34 bytes per parameter at 6.5 TB/s (1.18 G parameters 6163 us).  A
+// resident grid striding over the whole buffer kept nine streams apart by a grid's width each: 6825 us, and 6674 with two
+// vectors per thread in flight.
+constexpr int ADAM_UNROLL = 2;
+
+__global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float* __restrict__ g,
                              bf16* __restrict__ shadow, long long n, float lr, float b1, float b2, float eps, float wd,
                              float inv_bc1, float inv_bc2, const float* __restrict__ gscale, int zero_grad) {
   const float gs = gscale != nullptr ? *gscale : 1.f;
   const long long n4 = n / 4;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+  const long long span = (long long)blockDim.x * ADAM_UNROLL;
+  for (long long i0 = blockIdx.x * span + threadIdx.x; i0 < n4; i0 += gridDim.x * span) {
     // streaming accesses: nothing of the optimizer state is read again before it has left the L2
-    float4 pv = __ldcs(reinterpret_cast<const float4*>(p) + i);
-    float4 mv = __ldcs(reinterpret_cast<const float4*>(m) + i);
-    float4 vv = __ldcs(reinterpret_cast<const float4*>(v) + i);
-    float4 gv = __ldcs(reinterpret_cast<const float4*>(g) + i);
-    float pa[4] = {pv.x, pv.y, pv.z, pv.w}, ma[4] = {mv.x, mv.y, mv.z, mv.w}, va[4] = {vv.x, vv.y, vv.z, vv.w},
-          ga[4] = {gv.x, gv.y, gv.z, gv.w};
+    float4 pv[ADAM_UNROLL], mv[ADAM_UNROLL], vv[ADAM_UNROLL], gv[ADAM_UNROLL];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float gg = ga[j] * gs;
-      ma[j] = b1 * ma[j] + (1.f - b1) * gg;
-      va[j] = b2 * va[j] + (1.f - b2) * gg * gg;
-      const float mh = ma[j] * inv_bc1, vh = va[j] * inv_bc2;
-      pa[j] -= lr * (mh / (sqrtf(vh) + eps) + wd * pa[j]);
+    for (int k = 0; k < ADAM_UNROLL; ++k) {
+      const long long i = i0 + k * (long long)blockDim.x;
+      if (i < n4) {
+        pv[k] = __ldcs(reinterpret_cast<const float4*>(p) + i);
+        mv[k] = __ldcs(reinterpret_cast<const float4*>(m) + i);
+        vv[k] = __ldcs(reinterpret_cast<const float4*>(v) + i);
+        gv[k] = __ldcs(reinterpret_cast<const float4*>(g) + i);
+      }
     }
-    __stcs(reinterpret_cast<float4*>(p) + i, make_float4(pa[0], pa[1], pa[2], pa[3]));
-    __stcs(reinterpret_cast<float4*>(m) + i, make_float4(ma[0], ma[1], ma[2], ma[3]));
-    __stcs(reinterpret_cast<float4*>(v) + i, make_float4(va[0], va[1], va[2], va[3]));
-    if (zero_grad) __stcs(reinterpret_cast<float4*>(g) + i, make_float4(0.f, 0.f, 0.f, 0.f));
-    if (shadow != nullptr) {
-      uint2 s;
-      s.x = pack_bf16x2(pa[0], pa[1]);
-      s.y = pack_bf16x2(pa[2], pa[3]);
-      __stcs(reinterpret_cast<uint2*>(shadow) + i, s);
+#pragma unroll
+    for (int k = 0; k < ADAM_UNROLL; ++k) {
+      const long long i = i0 + k * (long long)blockDim.x;
+      if (i >= n4) break;
+      float pa[4] = {pv[k].x, pv[k].y, pv[k].z, pv[k].w}, ma[4] = {mv[k].x, mv[k].y, mv[k].z, mv[k].w},
+            va[4] = {vv[k].x, vv[k].y, vv[k].z, vv[k].w}, ga[4] = {gv[k].x, gv[k].y, gv[k].z, gv[k].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float gg = ga[j] * gs;
+        ma[j] = b1 * ma[j] + (1.f - b1) * gg;
+        va[j] = b2 * va[j] + (1.f - b2) * gg * gg;
+        const float mh = ma[j] * inv_bc1, vh = va[j] * inv_bc2;
+        pa[j] -= lr * (mh / (sqrtf(vh) + eps) + wd * pa[j]);
+      }
+      __stcs(reinterpret_cast<float4*>(p) + i, make_float4(pa[0], pa[1], pa[2], pa[3]));
+      __stcs(reinterpret_cast<float4*>(m) + i, make_float4(ma[0], ma[1], ma[2], ma[3]));
+      __stcs(reinterpret_cast<float4*>(v) + i, make_float4(va[0], va[1], va[2], va[3]));
+      if (zero_grad) __stcs(reinterpret_cast<float4*>(g) + i, make_float4(0.f, 0.f, 0.f, 0.f));
+      if (shadow != nullptr) {
+        uint2 s;
+        s.x = pack_bf16x2(pa[0], pa[1]);
+        s.y = pack_bf16x2(pa[2], pa[3]);
+        __stcs(reinterpret_cast<uint2*>(shadow) + i, s);
+      }
     }
   }
   // tail (n not a multiple of 4)
@@ -461,7 +481,7 @@ extern "C" int ob_adamw(float* p, float* m, float* v, float* g, void* shadow, lo
                         float eps, float wd, float bias_corr1, float bias_corr2, const float* gscale, int zero_grad,
                         cudaStream_t stream) {
   if (n <= 0) return 0;
-  adamw_kernel<<<blocks_for((n + 3) / 4, 256, 8), 256, 0, stream>>>(p, m, v, g, (bf16*)shadow, n, lr, b1, b2, eps, wd,
+  adamw_kernel<<<blocks_for((n + 3) / 4, 256 * ADAM_UNROLL, INT_MAX / 4096), 256, 0, stream>>>(p, m, v, g, (bf16*)shadow, n, lr, b1, b2, eps, wd,
                                                                     1.f / bias_corr1, 1.f / bias_corr2, gscale, zero_grad);
   OB_CUDA_OK(cudaGetLastError());
   return 0;

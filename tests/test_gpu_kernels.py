@@ -794,6 +794,21 @@ def test_cross_entropy_row_lengths(K, rows, V, softcap):
     _check_status()
 
 
+@pytest.mark.parametrize("n", [1, 3, 2047, 2048, 2052, 5 * 2048 + 1027])   # one block takes 2 x 256 vectors of four
+def test_adamw_lengths(K, n):
+    torch.manual_seed(n)
+    p, m, v, g = (torch.randn(n, device="cuda") for _ in range(4))
+    v = v.abs()
+    want_m, want_v = 0.9 * m + 0.1 * g, 0.95 * v + 0.05 * g * g
+    want_p = p - 1e-2 * ((want_m / 0.5) / ((want_v / 0.25).sqrt() + 1e-8) + 0.1 * p)
+    shadow = torch.zeros(n, device="cuda", dtype=torch.bfloat16)
+    K.adamw(p, m, v, g, shadow, lr=1e-2, b1=0.9, b2=0.95, eps=1e-8, wd=0.1, bias_corr1=0.5, bias_corr2=0.25, zero_grad=True)
+    for got, want in ((p, want_p), (m, want_m), (v, want_v)):
+        assert rel_err(got, want) < 1e-6   # a handful of fp32 roundings
+    assert torch.equal(shadow, p.to(torch.bfloat16)) and not g.any()
+    _check_status()
+
+
 def test_adamw_and_norm_kernels(K):
     dev = "cuda"
     torch.manual_seed(8)
