@@ -7,6 +7,9 @@
 // reference's "upcast, compute, cast back" rule (`olmax/nn/functional.py:51-67`, `olmax/nn/rope.py:99-115`,
 // `olmax/nn/mlp.py:69-73`, `olmax/nn/embedding.py:30-32`).
 #include "elementwise.h"
+
+#include <atomic>
+
 #include "host_common.h"
 #include "sm100.cuh"
 
@@ -769,12 +772,24 @@ using namespace ob;
 
 // Grid of a grid-stride normalisation kernel: exactly the number of blocks that are resident at once (occupancy x
 // SMs), never more -- a second, partly filled wave of blocks would run at a fraction of the memory parallelism.
-template <typename Kernel>
-static inline int resident_grid(Kernel kernel, long long work_blocks, size_t smem) {
+// The occupancy of a kernel (it depends on the device and the shared memory only) is asked for once and kept.
+template <auto KERNEL>
+static inline int resident_grid(long long work_blocks, size_t smem) {
+  static std::atomic<unsigned long long> known[64];   // per device: shared memory (high half), blocks per SM (low half)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NORM_THREADS, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  long long cap = (long long)sm_count() * per_sm;
+  if (dev >= 0 && dev < 64) {
+    const unsigned long long k = known[dev].load(std::memory_order_relaxed);
+    if ((k >> 32) == smem) per_sm = (int)(k & 0xffffffffu);
+  }
+  if (per_sm < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, NORM_THREADS, smem) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    else if (dev >= 0 && dev < 64)
+      known[dev].store((unsigned long long)smem << 32 | (unsigned)per_sm, std::memory_order_relaxed);
+  }
+  const long long cap = (long long)sm_count() * per_sm;
   return (int)(work_blocks < cap ? (work_blocks < 1 ? 1 : work_blocks) : cap);
 }
 
@@ -810,8 +825,8 @@ extern "C" int ob_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
   return norm_dispatch(d, "rmsnorm", [&](auto shape) {
     using S = decltype(shape);
     const int rpb = NORM_THREADS / S::TPR;
-    auto kernel = rmsnorm_fwd_kernel<S::TPR, S::VPT>;
-    kernel<<<resident_grid(kernel, (rows + rpb - 1) / rpb, 0), NORM_THREADS, 0, stream>>>(
+    constexpr auto kernel = rmsnorm_fwd_kernel<S::TPR, S::VPT>;
+    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, 0), NORM_THREADS, 0, stream>>>(
         (const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)sum_out, rstd, rows, d, heads, ld_x, ld_res,
         ld_y, add_before, eps);
   });
@@ -825,8 +840,8 @@ extern "C" int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   return norm_dispatch(d, "rmsnorm", [&](auto shape) {
     using S = decltype(shape);
     const int rpb = NORM_THREADS / S::TPR;
-    auto kernel = rmsnorm_bwd_kernel<S::TPR, S::VPT>;
-    kernel<<<resident_grid(kernel, (rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
+    constexpr auto kernel = rmsnorm_bwd_kernel<S::TPR, S::VPT>;
+    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
         (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dsum, (bf16*)dx, dw, rows, d, heads, ld_dy,
         ld_x, ld_dx, dw_scale);
   });
@@ -839,8 +854,8 @@ extern "C" int ob_layernorm_fwd(const void* x, const void* w, const void* b, voi
   return norm_dispatch(d, "layernorm", [&](auto shape) {
     using S = decltype(shape);
     const int rpb = NORM_THREADS / S::TPR;
-    auto kernel = layernorm_fwd_kernel<S::TPR, S::VPT>;
-    kernel<<<resident_grid(kernel, (rows + rpb - 1) / rpb, 0), NORM_THREADS, 0, stream>>>(
+    constexpr auto kernel = layernorm_fwd_kernel<S::TPR, S::VPT>;
+    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, 0), NORM_THREADS, 0, stream>>>(
         (const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, rows, d, eps);
   });
 }
@@ -855,8 +870,8 @@ extern "C" int ob_layernorm_bwd(const void* dy, const void* x, const void* w, co
     const int rpb = NORM_THREADS / S::TPR;
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(layernorm_bwd_kernel<S::TPR, S::VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    auto kernel = layernorm_bwd_kernel<S::TPR, S::VPT>;
-    kernel<<<resident_grid(kernel, (rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
+    constexpr auto kernel = layernorm_bwd_kernel<S::TPR, S::VPT>;
+    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
         (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd, (bf16*)dx, dw, db, rows, d, scale);
   });
 }
@@ -898,8 +913,8 @@ extern "C" int ob_rmsnorm_rope_fwd(const void* x, const void* w, void* y, float*
   return norm_rope_dispatch(d, hd, "rmsnorm_rope", [&](auto shape) {
     using Sh = decltype(shape);
     const int rpb = NORM_THREADS / Sh::TPR;
-    auto kernel = rmsnorm_rope_fwd_kernel<Sh::TPR, Sh::VPT>;
-    kernel<<<resident_grid(kernel, (rows + rpb - 1) / rpb, 0), NORM_THREADS, 0, stream>>>(
+    constexpr auto kernel = rmsnorm_rope_fwd_kernel<Sh::TPR, Sh::VPT>;
+    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, 0), NORM_THREADS, 0, stream>>>(
         (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, cos_t, sin_t, rows, d, hd, heads, ld_x, ld_y, S, eps);
   });
 }
@@ -914,8 +929,8 @@ extern "C" int ob_rmsnorm_rope_bwd(const void* dy, const void* x, const void* w,
   return norm_rope_dispatch(d, hd, "rmsnorm_rope", [&](auto shape) {
     using Sh = decltype(shape);
     const int rpb = NORM_THREADS / Sh::TPR;
-    auto kernel = rmsnorm_rope_bwd_kernel<Sh::TPR, Sh::VPT>;
-    kernel<<<resident_grid(kernel, (rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
+    constexpr auto kernel = rmsnorm_rope_bwd_kernel<Sh::TPR, Sh::VPT>;
+    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
         (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (bf16*)dx, dw, cos_t, sin_t, rows, d, hd, heads, ld_dy,
         ld_x, ld_dx, S, dw_scale);
   });

@@ -141,8 +141,10 @@ def check(rc: int, what: str) -> None:
         raise KernelError(f"{what} failed (code {rc}): {msg.decode() if msg else ''}")
 
 
-def stream_ptr(device: Optional[torch.device] = None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def stream_ptr(device: Optional[torch.device] = None) -> int:
+    """Handle of the current stream of ``device`` (default: the current device), without building a Stream object."""
+    index = device.index if device is not None else None
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 _STATUS: dict = {}

@@ -152,29 +152,36 @@ def gemm(
     args.lda = lda if lda is not None else a.stride(0)
     args.b = b.data_ptr()
     args.ldb = ldb if ldb is not None else b.stride(0)
-    args.b_shard_stride = b_shard_stride
-    args.b2 = _ptr(b2)
     args.c = c.data_ptr()
     args.ldc = ldc if ldc is not None else c.stride(0)
-    args.c2 = _ptr(c2)
-    args.c3 = _ptr(c3)
-    args.c_shards = _ptr(c_shards)
-    args.c_shard_stride = c_shard_stride
     args.M, args.N, args.Kc = M, N, K
-    args.M_s, args.N_s, args.Kc_s = M_s, N_s, Kc_s
     args.a_mn, args.b_mn, args.epi, args.alpha = int(a_mn), int(b_mn), epi, alpha
     args.status = status_buffer(a.device).data_ptr()
-    args.max_ctas = max_ctas
-    args.ag_src = _ptr(ag_src)
-    args.ag_src2 = _ptr(ag_src2)
-    args.ag_flags = _ptr(ag_flags)
-    args.ag_rank = ag_rank
-    args.no_tma_epilogue = int(no_tma_epilogue)
-    args.group_m = group_m
-    args.m_shard_rot = m_shard_rot
-    args.multi_box_mn = int(multi_box_mn)
-    args.ag_on_a = int(ag_on_a)
-    args.no_split_k = int(no_split_k)
+    # (a new struct is all zeros: what few calls use is filled in only where it is given)
+    if b2 is not None:
+        args.b2 = b2.data_ptr()
+    if c2 is not None:
+        args.c2 = c2.data_ptr()
+    if c3 is not None:
+        args.c3 = c3.data_ptr()
+    if N_s or Kc_s or M_s or b_shard_stride or c_shard_stride or c_shards is not None:
+        args.M_s, args.N_s, args.Kc_s = M_s, N_s, Kc_s
+        args.b_shard_stride = b_shard_stride
+        args.c_shard_stride = c_shard_stride
+        args.c_shards = _ptr(c_shards)
+    if ag_src is not None:
+        args.ag_src = ag_src.data_ptr()
+        args.ag_src2 = _ptr(ag_src2)
+        args.ag_flags = _ptr(ag_flags)
+        args.ag_rank = ag_rank
+        args.ag_on_a = int(ag_on_a)
+    if max_ctas or no_tma_epilogue or group_m or m_shard_rot or multi_box_mn or no_split_k:
+        args.max_ctas = max_ctas
+        args.no_tma_epilogue = int(no_tma_epilogue)
+        args.group_m = group_m
+        args.m_shard_rot = m_shard_rot
+        args.multi_box_mn = int(multi_box_mn)
+        args.no_split_k = int(no_split_k)
     if seg != SEG_NONE:
         pieces = (c if seg == SEG_C_N else a, *seg_rest)
         if not 2 <= len(pieces) <= 3 or any(t.stride(-1) != 1 for t in pieces):
@@ -193,14 +200,19 @@ def gemm(
     _count()
 
 
-def _set_bshd(args: ObAttnArgs, field: str, t: torch.Tensor, prefix: Optional[str] = None) -> None:
-    prefix = prefix or field
-    if t.stride(-1) != 1:
+_BSHD = {f: (f, *((f if f != "d_o" else "do") + s for s in ("_sb", "_ss", "_sh")))
+         for f in ("q", "k", "v", "o", "d_o", "dq", "dk", "dv")}
+
+
+def _set_bshd(args: ObAttnArgs, field: str, t: torch.Tensor) -> None:
+    ptr, sb, ss, sh = _BSHD[field]
+    strides = t.stride()
+    if strides[-1] != 1:
         raise KernelError("attention tensors need a contiguous head dimension")
-    setattr(args, field, t.data_ptr())
-    setattr(args, prefix + "_sb", t.stride(0))
-    setattr(args, prefix + "_ss", t.stride(1))
-    setattr(args, prefix + "_sh", t.stride(2))
+    setattr(args, ptr, t.data_ptr())
+    setattr(args, sb, strides[0])
+    setattr(args, ss, strides[1])
+    setattr(args, sh, strides[2])
 
 
 def flash_attn_fwd(q, k, v, *, causal=True, window=-1, softcap=0.0, scale=None, q_off=0) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -241,7 +253,7 @@ def flash_attn_bwd(q, k, v, o, lse, d_o, *, causal=True, window=-1, softcap=0.0,
     _set_bshd(a, "k", k)
     _set_bshd(a, "v", v)
     _set_bshd(a, "o", o)
-    _set_bshd(a, "d_o", d_o, "do")
+    _set_bshd(a, "d_o", d_o)
     _set_bshd(a, "dq", dq)
     _set_bshd(a, "dk", dk)
     _set_bshd(a, "dv", dv)

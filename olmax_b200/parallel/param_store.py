@@ -107,9 +107,15 @@ class ParamHandle:
         """(rank-0 piece view, element stride between consecutive ranks' pieces) of the gathered weight."""
         assert self.unit is not None
         buf = self.unit.gathered()
+        return self._piece_view(buf), buf.stride(0)
+
+    def _piece_view(self, buf: torch.Tensor) -> torch.Tensor:
+        """This parameter's rank-0 piece of a ``[R, unit_numel]`` buffer, as one view."""
         m = self.meta
-        first = buf[0, m.unit_offset : m.unit_offset + m.numel_local].view(m.local_shape)
-        return first, buf.stride(0)
+        if len(m.local_shape) > 2:
+            return buf[0, m.unit_offset : m.unit_offset + m.numel_local].view(m.local_shape)
+        strides = (m.local_shape[1], 1) if len(m.local_shape) == 2 else (1,)
+        return buf.as_strided(m.local_shape, strides, buf.storage_offset() + m.unit_offset)
 
     def full(self) -> torch.Tensor:
         """The TP-local weight in compute dtype, assembled from the gathered unit (a view when the group is 1)."""
@@ -118,7 +124,7 @@ class ParamHandle:
         m = self.meta
         buf = self.unit.gathered()
         if R == 1:
-            return buf[0, m.unit_offset : m.unit_offset + m.numel_local].view(m.local_shape)
+            return self._piece_view(buf)
         cached = self.unit._full_cache.get(m.name)
         if cached is None:
             if m.name in self.unit._ag_pending:
