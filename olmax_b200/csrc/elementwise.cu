@@ -8,6 +8,8 @@
 // `olmax/nn/mlp.py:69-73`, `olmax/nn/embedding.py:30-32`).
 #include "elementwise.h"
 
+#include <limits.h>
+
 #include <atomic>
 
 #include "host_common.h"
@@ -948,7 +950,9 @@ extern "C" int ob_glu_bwd(const void* g, const void* u, const void* da, void* dg
                           int gelu, cudaStream_t stream) {
   if (n % 8 != 0) OB_FAIL(-1, "glu: element count must be a multiple of 8");
   if (n == 0) return 0;
-  glu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>((const bf16*)g, (const bf16*)u, (const bf16*)da, (bf16*)dg,
+  // one block per 256 vectors, in launch order: six streams at 6.8 TB/s (65536 x 2816: 325 us); a resident grid striding over
+  // the whole tensors took 393 us, and 417 with GeGLU
+  glu_bwd_kernel<<<grid_for(n / 8, 256, INT_MAX / 4096), 256, 0, stream>>>((const bf16*)g, (const bf16*)u, (const bf16*)da, (bf16*)dg,
                                                            (bf16*)du, (bf16*)a_out, n / 8, gelu);
   OB_CUDA_OK(cudaGetLastError());
   return 0;
