@@ -638,21 +638,15 @@ __global__ void __launch_bounds__(NORM_THREADS, PPT <= 1 ? 3 : 2)
   for (int i = threadIdx.x; i < d; i += NORM_THREADS) atomicAdd(dw + i, dw_part[i] * dw_scale);
 }
 
-// x * sigmoid(z), as in the gated GEMM's epilogue (the backward pass rebuilds the value that the forward pass rounded)
-__device__ __forceinline__ float gelu_tanh_arg(float x) {   // 2 u: gelu_tanh(x) = x * sigmoid(2 u)
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 2.f * (k0 * (x + k1 * x * x * x));
-}
-__device__ __forceinline__ float sigmoid_fast(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
-__device__ __forceinline__ float act_silu(float x) { return x * sigmoid_fast(x); }
+__device__ __forceinline__ float act_silu(float x) { return x * silu_sigmoid(x); }
 __device__ __forceinline__ float act_silu_grad(float x) {
-  const float s = sigmoid_fast(x);
+  const float s = silu_sigmoid(x);
   return s * (1.f + x * (1.f - s));
 }
-__device__ __forceinline__ float act_gelu_tanh(float x) { return x * sigmoid_fast(gelu_tanh_arg(x)); }
+__device__ __forceinline__ float act_gelu_tanh(float x) { return x * gelu_sigmoid(x); }
 __device__ __forceinline__ float act_gelu_tanh_grad(float x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float s = sigmoid_fast(gelu_tanh_arg(x));
+  const float s = gelu_sigmoid(x);
   return s + 2.f * x * s * (1.f - s) * k0 * (1.f + 3.f * k1 * x * x);
 }
 

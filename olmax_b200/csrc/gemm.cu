@@ -175,16 +175,13 @@ __device__ __forceinline__ bool ag_wait(const KernelParams& p, int shard, int bl
   return false;
 }
 
-// Both activations as x * sigmoid(z) = x / (1 + exp(-z)): gelu_tanh(x) = 0.5 x (1 + tanh(u)) is x * sigmoid(2 u), without the
-// cancellation of 1 + tanh(u) for negative u.  No branches: the epilogue warp is alone on its scheduler, and a division or
-// tanhf with a slow path cuts the 16-element batch into basic blocks whose latencies no longer overlap (65536 x 2816 x 1024,
-// SwiGLU with both pre-activations: 1306 us with them, 898 without).
-__device__ __forceinline__ float gelu_tanh(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float u = k0 * (x + k1 * x * x * x);
-  return x * __fdividef(1.0f, 1.0f + __expf(-2.0f * u));
+// act(g) * u for two columns.  The epilogue warp is alone on its scheduler: a division or tanhf with a slow path cuts the batch
+// into basic blocks whose latencies no longer overlap, and every instruction counts (65536 x 2816 x 1024, SwiGLU with both
+// pre-activations and staged stores: 772 us with __expf and __fdividef, 580 us so; 1306 us with a division and
+// per-thread stores).
+__device__ __forceinline__ float2 gated2(bool swiglu, float2 g, float2 u) {
+  return mul2(mul2(g, swiglu ? silu_sigmoid2(g) : gelu_sigmoid2(g)), u);
 }
-__device__ __forceinline__ float silu(float x) { return x * __fdividef(1.0f, 1.0f + __expf(-x)); }
 
 // Work item w of a launch: a whole tile, or (in the split-K tail) one k slice of a tile.
 __device__ __forceinline__ void decode_work(const KernelParams& p, int w, int k_iters, int& tile, int& k_begin, int& k_count) {
@@ -555,7 +552,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         // Gated epilogue, columns [0, 128) = gate, [128, 256) = up: 64 output columns at a time, the activation and (when
         // kept for the backward pass) the two pre-activations staged one after the other and stored by TMA.  With a k loop
         // of 16 iterations this epilogue is longer than the main loop: 65536 x 2816 x 1024 (three outputs) took 898 us with
-        // per-thread 16-byte stores, 772 us so; 1000 x 2816 x 1024 37 -> 33 us.
+        // per-thread 16-byte stores, 772 us so, both with the activations as they were then (580 us with those of today).
         const bool store_thread = (threadIdx.x == 64);
         const int sw = row_in_tile & 7;
         auto stage = [&](const CUtensorMap* map, const uint32_t (&w)[32], int col) {
@@ -573,6 +570,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             tma_store_commit();
           }
         };
+        const bool swiglu = p.epi == EPI_SWIGLU;
         for (int c0 = 0; c0 < 128 && c0 < n_valid; c0 += 64) {
           uint32_t va[32], vg[32], vu[32];
 #pragma unroll
@@ -587,8 +585,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               vg[h * 8 + j] = pack_bf16x2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
               vu[h * 8 + j] = pack_bf16x2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
               const float2 gf = unpack_bf16x2(vg[h * 8 + j]), uf = unpack_bf16x2(vu[h * 8 + j]);
-              va[h * 8 + j] = p.epi == EPI_SWIGLU ? pack_bf16x2(silu(gf.x) * uf.x, silu(gf.y) * uf.y)
-                                                  : pack_bf16x2(gelu_tanh(gf.x) * uf.x, gelu_tanh(gf.y) * uf.y);
+              const float2 af = gated2(swiglu, gf, uf);
+              va[h * 8 + j] = pack_bf16x2(af.x, af.y);
             }
           }
           stage(&tmC, va, n_glob0 + c0);
@@ -789,11 +787,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             const int nv = min(16, n_valid - c0);
             float a[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < 16; j += 2) {
               // round gate / up to bf16 first so that act(g)*u matches what a backward pass recomputes from them
-              float gf = __bfloat162float(__float2bfloat16(__uint_as_float(g[j])));
-              float uf = __bfloat162float(__float2bfloat16(__uint_as_float(u[j])));
-              a[j] = (p.epi == EPI_SWIGLU ? silu(gf) : gelu_tanh(gf)) * uf;
+              const float2 gf = unpack_bf16x2(pack_bf16x2(__uint_as_float(g[j]), __uint_as_float(g[j + 1])));
+              const float2 uf = unpack_bf16x2(pack_bf16x2(__uint_as_float(u[j]), __uint_as_float(u[j + 1])));
+              const float2 af = gated2(p.epi == EPI_SWIGLU, gf, uf);
+              a[j] = af.x;
+              a[j + 1] = af.y;
             }
             const long long off = row_off + c0;
 #pragma unroll
@@ -993,7 +993,7 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     // 128 x 64 tiles, where all of them run at once and most pairs would have no 256 x 256 tile.  Their k-blocks come at the
     // same pace (about 280 ns, bound by the latency of the loads through eight stages), but they start and drain sooner:
     // 328 x 1024 x 2816 20.5 us against 26.7 with 128 x 256 single-CTA tiles, 1000 x 1024 x 5632 35 against 43, 1024 x
-    // 512 x 512 12.3 against 14.3.  In more than one wave they lose (2048 x 1024 x 50304: 533 us against @LM@ with pairs),
+    // 512 x 512 12.3 against 14.3.  In more than one wave they lose (2048 x 1024 x 50304: 533 us against 240 with pairs),
     // and to k slices on pairs where the contraction is long enough to be cut.
     if (!sharded && !glu && tiles(BM, BN_WIDE) <= cap / 2 && tiles(BM, BN_NARROW) <= cap &&
         !(split_ok && best_split((int)pair_tiles, cap / 2, k_iters_total).split > 1)) {
