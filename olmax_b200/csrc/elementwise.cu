@@ -402,35 +402,44 @@ __global__ void __launch_bounds__(NORM_THREADS)
 }
 
 // Rotary embedding, rotate-half convention: out = x * cos + rotate_half(x) * sin, cos/sin tables [S, D/2] fp32.
-// sign = +1 forward, -1 backward (the transpose of a rotation).  One thread per 8 elements of the first half.
-__global__ void rope_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ cos_t,
-                            const float* __restrict__ sin_t, int B, int S, int H, int D, long long sb, long long ss,
-                            long long sh, long long ysb, long long yss, long long ysh, float sign, int pos_offset) {
-  const int half = D / 2;
-  const int vec_per_head = half / 8;
-  const long long total = (long long)B * S * H * vec_per_head;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int vi = (int)(idx % vec_per_head);
-    const int h = (int)((idx / vec_per_head) % H);
-    const int s = (int)((idx / ((long long)vec_per_head * H)) % S);
-    const int b = (int)(idx / ((long long)vec_per_head * H * S));
-    const bf16* px = x + b * sb + s * ss + h * sh + vi * 8;
-    bf16* py = y + b * ysb + s * yss + h * ysh + vi * 8;
-    float lo[8], hi[8], c[8], sn[8], olo[8], ohi[8];
-    load8(px, lo);
-    load8(px + half, hi);
-    load8f(cos_t + (long long)(s + pos_offset) * half + vi * 8, c);
-    load8f(sin_t + (long long)(s + pos_offset) * half + vi * 8, sn);
+// sign = +1 forward, -1 backward (the transpose of a rotation).  One thread per 8 elements of the first half.  A launch
+// takes one tensor or two that share batch, positions and tables (q and k: the first `a_blocks` blocks work on the first).
+// Bound by HBM for long sequences (5.2 TB/s) and by the launch for short ones.
+struct RopeTensor {
+  const bf16* x;
+  bf16* y;
+  int H;
+  long long sb, ss, sh, ysb, yss, ysh;
+};
+
+template <typename I>
+__global__ void __launch_bounds__(256)
+    rope_kernel(const RopeTensor ta, const RopeTensor tb, unsigned a_blocks, const float* __restrict__ cos_t,
+                const float* __restrict__ sin_t, int B, int S, int D, float sign, int pos_offset) {
+  const bool second = blockIdx.x >= a_blocks;
+  const RopeTensor& t = second ? tb : ta;
+  const int half = D / 2, vec_per_head = half / 8;
+  const I total = (I)B * (I)S * (I)t.H * (I)vec_per_head;
+  const I idx = (I)(blockIdx.x - (second ? a_blocks : 0)) * 256 + threadIdx.x;
+  if (idx >= total) return;
+  const I bsh = idx / (I)vec_per_head, bs = bsh / (I)t.H;
+  const int vi = (int)(idx - bsh * (I)vec_per_head), h = (int)(bsh - bs * (I)t.H);
+  const int b = (int)(bs / (I)S), s = (int)(bs - (I)b * (I)S);
+  const bf16* px = t.x + b * t.sb + s * t.ss + h * t.sh + vi * 8;
+  bf16* py = t.y + b * t.ysb + s * t.yss + h * t.ysh + vi * 8;
+  float lo[8], hi[8], c[8], sn[8], olo[8], ohi[8];
+  load8(px, lo);
+  load8(px + half, hi);
+  load8f(cos_t + (long long)(s + pos_offset) * half + vi * 8, c);
+  load8f(sin_t + (long long)(s + pos_offset) * half + vi * 8, sn);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sj = sn[j] * sign;
-      olo[j] = lo[j] * c[j] - hi[j] * sj;
-      ohi[j] = hi[j] * c[j] + lo[j] * sj;
-    }
-    store8(py, olo);
-    store8(py + half, ohi);
+  for (int j = 0; j < 8; ++j) {
+    const float sj = sn[j] * sign;
+    olo[j] = lo[j] * c[j] - hi[j] * sj;
+    ohi[j] = hi[j] * c[j] + lo[j] * sj;
   }
+  store8(py, olo);
+  store8(py + half, ohi);
 }
 
 // q / k normalisation fused with the rotary embedding:  y = rope(rmsnorm(x) * w).
@@ -872,16 +881,37 @@ extern "C" int ob_layernorm_bwd(const void* dy, const void* x, const void* w, co
   });
 }
 
+static int launch_rope(const RopeTensor& a, const RopeTensor& b, const float* cos_t, const float* sin_t, int B, int S, int D,
+                       float sign, int pos_offset, cudaStream_t stream) {
+  if (D % 16 != 0) OB_FAIL(-1, "rope: head dim (%d) must be a multiple of 16", D);
+  const long long na = (long long)B * S * a.H * (D / 16), nb = (long long)B * S * b.H * (D / 16);
+  if (na < 0 || nb < 0 || na + nb == 0) return 0;
+  const long long ba = (na + 255) / 256, bb = (nb + 255) / 256;
+  if (ba + bb > INT_MAX) OB_FAIL(-2, "rope: %lld vectors exceed the grid", na + nb);
+  if (na < INT_MAX && nb < INT_MAX)
+    rope_kernel<unsigned><<<(unsigned)(ba + bb), 256, 0, stream>>>(a, b, (unsigned)ba, cos_t, sin_t, B, S, D, sign, pos_offset);
+  else
+    rope_kernel<unsigned long long><<<(unsigned)(ba + bb), 256, 0, stream>>>(a, b, (unsigned)ba, cos_t, sin_t, B, S, D, sign, pos_offset);
+  OB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
 extern "C" int ob_rope(const void* x, void* y, const float* cos_t, const float* sin_t, int B, int S, int H, int D,
                        long long sb, long long ss, long long sh, long long ysb, long long yss, long long ysh,
                        float sign, int pos_offset, cudaStream_t stream) {
-  if (D % 16 != 0) OB_FAIL(-1, "rope: head dim (%d) must be a multiple of 16", D);
-  const long long total = (long long)B * S * H * (D / 16);
-  if (total <= 0) return 0;
-  rope_kernel<<<grid_for(total, 256), 256, 0, stream>>>((const bf16*)x, (bf16*)y, cos_t, sin_t, B, S, H, D, sb, ss, sh,
-                                                        ysb, yss, ysh, sign, pos_offset);
-  OB_CUDA_OK(cudaGetLastError());
-  return 0;
+  const RopeTensor t{(const bf16*)x, (bf16*)y, H, sb, ss, sh, ysb, yss, ysh};
+  RopeTensor none = t;
+  none.H = 0;
+  return launch_rope(t, none, cos_t, sin_t, B, S, D, sign, pos_offset, stream);
+}
+
+extern "C" int ob_rope_pair(const void* x1, void* y1, int H1, long long sb1, long long ss1, long long sh1, long long ysb1,
+                            long long yss1, long long ysh1, const void* x2, void* y2, int H2, long long sb2, long long ss2,
+                            long long sh2, long long ysb2, long long yss2, long long ysh2, const float* cos_t,
+                            const float* sin_t, int B, int S, int D, float sign, cudaStream_t stream) {
+  const RopeTensor a{(const bf16*)x1, (bf16*)y1, H1, sb1, ss1, sh1, ysb1, yss1, ysh1};
+  const RopeTensor b{(const bf16*)x2, (bf16*)y2, H2, sb2, ss2, sh2, ysb2, yss2, ysh2};
+  return launch_rope(a, b, cos_t, sin_t, B, S, D, sign, 0, stream);
 }
 
 // Thread layout of the fused norm + rotary kernels for a row of d / 16 pairs.

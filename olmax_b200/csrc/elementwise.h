@@ -27,6 +27,11 @@ int ob_layernorm_bwd(const void* dy, const void* x, const void* w, const float* 
 int ob_rope(const void* x, void* y, const float* cos_t, const float* sin_t, int B, int S, int H, int D, long long sb,
             long long ss, long long sh, long long ysb, long long yss, long long ysh, float sign, int pos_offset,
             cudaStream_t stream);
+// the same for two tensors that share batch, positions and tables (q and k), in one launch
+int ob_rope_pair(const void* x1, void* y1, int H1, long long sb1, long long ss1, long long sh1, long long ysb1, long long yss1,
+                 long long ysh1, const void* x2, void* y2, int H2, long long sb2, long long ss2, long long sh2, long long ysb2,
+                 long long yss2, long long ysh2, const float* cos_t, const float* sin_t, int B, int S, int D, float sign,
+                 cudaStream_t stream);
 // y = rope(rmsnorm(x) * w) in one pass (q / k normalisation followed by the rotary embedding).  A row of d
 // elements is d / hd heads; rows are addressed like ob_rmsnorm_fwd; the table row of a row is (row / heads) % S.
 int ob_rmsnorm_rope_fwd(const void* x, const void* w, void* y, float* rstd, const float* cos_t, const float* sin_t,

@@ -23,7 +23,7 @@ from ..types import StrEnum
 from .linear import Linear, linear_group
 from .module import Module, current_build_context
 from .normalization import NormalizerConfig, RMSNorm, RMSNormConfig
-from .rope import BufferCache, RotaryPositionalEmbedding, RotaryPositionalEmbeddingConfig
+from .rope import BufferCache, RotaryPositionalEmbedding, RotaryPositionalEmbeddingConfig, rotate_qk
 
 __all__ = ["AttentionImplementation", "AttentionKernel", "MultiheadSelfAttention", "MultiheadSelfAttentionConfig"]
 
@@ -147,8 +147,7 @@ class MultiheadSelfAttention(Module):
             k = k.view(batch_size, S, self.local_kv_heads, self.head_dim)
             if self.rope is not None:
                 cp = self.mesh.cp
-                q = self.rope(q, cache, cp.size, cp.rank)
-                k = self.rope(k, cache, cp.size, cp.rank)
+                q, k = rotate_qk(self.rope, q, k, cache, cp.size, cp.rank)
         return q, k, v
 
     @property

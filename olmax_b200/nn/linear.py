@@ -9,7 +9,7 @@ import torch
 from ..ops import functional as F
 from ..parallel import collectives as coll
 from ..parallel.mesh import TPStyle
-from .module import Module
+from .module import Module, is_hooked
 
 __all__ = ["Linear", "linear_group"]
 
@@ -44,11 +44,6 @@ class Linear(Module):
 def linear_group(mods, x: torch.Tensor):
     """``m(x)`` for every module of a group that reads one input, as one GEMM where they are plain unhooked
     :class:`Linear` layers whose weights can be joined."""
-    if all(type(m) is Linear and "forward" not in m.__dict__ and not _hooked(m) for m in mods):
+    if all(type(m) is Linear and "forward" not in m.__dict__ and not is_hooked(m) for m in mods):
         return F.linears(x, [m.weight for m in mods], [m.bias for m in mods])
     return tuple(m(x) for m in mods)
-
-
-def _hooked(m: torch.nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                or torch.nn.modules.module._has_any_global_hook())

@@ -93,6 +93,12 @@ class Module(torch.nn.Module):
         return [m.checkpoint_name for m in self.modules() if isinstance(m, Module) and m.checkpoint_name]
 
 
+def is_hooked(m: torch.nn.Module) -> bool:
+    """Whether calling ``m`` runs hooks: then nothing may be computed past its ``__call__``."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or torch.nn.modules.module._has_any_global_hook())
+
+
 def build_module(factory, *, seed: int = 0, mesh=None, mesh_resource=None, param_dtype: torch.dtype = torch.float32,
                  compute_dtype: Optional[torch.dtype] = None, device: Optional[torch.device] = None,
                  comm_backend: Optional[str] = None, unit: str = "root"):

@@ -9,8 +9,9 @@ import torch
 
 from ..ops import functional as F
 from ..ops import reference as ref
+from .module import is_hooked
 
-__all__ = ["RotaryPositionalEmbedding", "RotaryPositionalEmbeddingConfig", "BufferCache"]
+__all__ = ["RotaryPositionalEmbedding", "RotaryPositionalEmbeddingConfig", "BufferCache", "rotate_qk"]
 
 
 class BufferCache(dict):
@@ -58,6 +59,16 @@ class RotaryPositionalEmbedding(torch.nn.Module):
         """x: [B, S, H, D] (S = this rank's tokens under context parallelism)."""
         cos, sin = self.tables_for(x.shape[1], x.device, cache, cp_size, cp_rank)
         return F.rope(x, cos, sin)
+
+
+def rotate_qk(rope: torch.nn.Module, q: torch.Tensor, k: torch.Tensor, cache: Optional[BufferCache] = None, cp_size: int = 1,
+              cp_rank: int = 0):
+    """``(rope(q), rope(k))`` of one attention block, as one launch where ``rope`` is a plain unhooked
+    :class:`RotaryPositionalEmbedding`."""
+    if type(rope) is not RotaryPositionalEmbedding or "forward" in rope.__dict__ or is_hooked(rope):
+        return rope(q, cache, cp_size, cp_rank), rope(k, cache, cp_size, cp_rank)
+    cos, sin = rope.tables_for(q.shape[1], q.device, cache, cp_size, cp_rank)
+    return F.rope_pair(q, k, cos, sin)
 
 
 @dataclass

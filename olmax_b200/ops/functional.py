@@ -23,7 +23,7 @@ from ..parallel import collectives as coll
 from . import reference as ref
 
 __all__ = [
-    "linear", "linears", "gated_mlp", "rms_norm", "layer_norm", "rope", "attention", "attention_block_fwd", "attention_block_bwd",
+    "linear", "linears", "gated_mlp", "rms_norm", "layer_norm", "rope", "rope_pair", "attention", "attention_block_fwd", "attention_block_bwd",
     "embedding", "linear_cross_entropy", "glu", "tp_column_linears", "tp_row_linear",
 ]
 
@@ -659,6 +659,35 @@ class _RopeFn(torch.autograd.Function):
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     """x: [B, S, H, D]; cos/sin fp32 [>= S, D/2]."""
     return _RopeFn.apply(x, cos, sin)
+
+
+class _RopePairFn(torch.autograd.Function):
+    """:class:`_RopeFn` of q and k in one launch per direction (GPU)."""
+
+    @staticmethod
+    def _rotate(q, k, cos, sin, sign):
+        yq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+        yk = torch.empty(k.shape, dtype=k.dtype, device=k.device)
+        K.rope_pair(q, k, yq, yk, cos, sin, sign=sign)
+        return yq, yk
+
+    @staticmethod
+    def forward(ctx, q, k, cos, sin):
+        ctx.save_for_backward(cos, sin)
+        return _RopePairFn._rotate(q, k, cos, sin, 1.0)
+
+    @staticmethod
+    def backward(ctx, dq, dk):
+        cos, sin = ctx.saved_tensors
+        dq, dk = (d if d.stride(-1) == 1 else d.contiguous() for d in (dq, dk))
+        return (*_RopePairFn._rotate(dq, dk, cos, sin, -1.0), None, None)
+
+
+def rope_pair(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
+    """``(rope(q), rope(k))`` of one attention block: q [B, S, Hq, D], k [B, S, Hk, D]."""
+    if q.is_cuda and _on_gpu(q) and _on_gpu(k):
+        return _RopePairFn.apply(q, k, cos, sin)
+    return rope(q, cos, sin), rope(k, cos, sin)
 
 
 class _RMSNormRopeFn(torch.autograd.Function):

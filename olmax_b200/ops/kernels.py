@@ -24,7 +24,7 @@ from ._lib import KernelError, ObAttnArgs, ObGemmArgs, check, lib, register_sign
 __all__ = [
     "EPI_BF16", "EPI_F32", "EPI_F32_ACC", "EPI_F32_RED", "EPI_SWIGLU", "EPI_GEGLU", "EPI_BF16_ACC",
     "SEG_NONE", "SEG_A_K", "SEG_A_M", "SEG_C_N",
-    "gemm", "flash_attn_fwd", "flash_attn_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rmsnorm_rope_fwd", "rmsnorm_rope_bwd", "rope", "glu_fwd", "glu_bwd",
+    "gemm", "flash_attn_fwd", "flash_attn_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rmsnorm_rope_fwd", "rmsnorm_rope_bwd", "rope", "rope_pair", "glu_fwd", "glu_bwd",
     "embed_gather", "embed_scatter", "ce_fwd_bwd", "ce_vp_stats", "ce_vp_grad", "count_valid", "adamw", "sumsq", "clip_coef", "cast_f32_bf16",
     "layernorm_fwd", "layernorm_bwd", "gather_shards", "scatter_add_shards", "allreduce_p2p", "allreduce_multimem",
     "peer_barrier", "peer_signal", "peer_wait", "copy_bytes", "push_copy", "fold_slots_bf16", "reduce_slots",
@@ -62,6 +62,7 @@ register_signature("ob_rmsnorm_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i
 register_signature("ob_layernorm_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _f, _vp])
 register_signature("ob_layernorm_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _f, _vp])
 register_signature("ob_rope", [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _vp])
+register_signature("ob_rope_pair", ([_vp, _vp, _i] + [_ll] * 6) * 2 + [_vp, _vp, _i, _i, _i, _f, _vp])
 register_signature("ob_rmsnorm_rope_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _ll, _ll, _i, _f, _vp])
 register_signature("ob_rmsnorm_rope_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _ll, _ll, _ll, _i, _f, _vp])
 register_signature("ob_glu_fwd", [_vp, _vp, _vp, _ll, _i, _vp])
@@ -334,6 +335,18 @@ def rope(x, y, cos, sin, *, sign=1.0, pos_offset=0) -> None:
     _count()
 
 
+def rope_pair(q, k, yq, yk, cos, sin, *, sign=1.0) -> None:
+    """:func:`rope` of two tensors of one batch and sequence, [B, S, Hq, D] and [B, S, Hk, D], in one launch."""
+    _req_bf16(q, k, yq, yk)
+    B, S, H, D = q.shape
+    if k.shape[:2] != (B, S) or k.shape[3] != D or yq.shape != q.shape or yk.shape != k.shape:
+        raise KernelError("rope_pair: q and k must share batch, sequence and head dimension")
+    check(lib().ob_rope_pair(q.data_ptr(), yq.data_ptr(), H, *q.stride()[:3], *yq.stride()[:3],
+                             k.data_ptr(), yk.data_ptr(), k.shape[2], *k.stride()[:3], *yk.stride()[:3],
+                             cos.data_ptr(), sin.data_ptr(), B, S, D, sign, stream_ptr(q.device)), "rope_pair")
+    _count()
+
+
 def glu_fwd(g, u, a, gelu: bool) -> None:
     _req_bf16(g, u, a)
     check(lib().ob_glu_fwd(g.data_ptr(), u.data_ptr(), a.data_ptr(), g.numel(), int(gelu), stream_ptr(g.device)), "glu_fwd")
@@ -581,7 +594,7 @@ def format_timing(report: dict, top: int = 40) -> str:
 
 for _name in ("gemm", "flash_attn_fwd", "flash_attn_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rmsnorm_rope_fwd",
               "rmsnorm_rope_bwd", "layernorm_fwd", "layernorm_bwd",
-              "rope", "glu_fwd", "glu_bwd", "embed_gather", "embed_scatter", "ce_fwd_bwd", "ce_vp_stats", "ce_vp_grad", "count_valid",
+              "rope", "rope_pair", "glu_fwd", "glu_bwd", "embed_gather", "embed_scatter", "ce_fwd_bwd", "ce_vp_stats", "ce_vp_grad", "count_valid",
               "adamw", "sumsq",
               "clip_coef", "cast_f32_bf16", "gather_shards", "scatter_add_shards", "allreduce_p2p", "allreduce_multimem",
               "copy_bytes", "push_copy", "fold_slots_bf16", "reduce_slots", "peer_barrier", "peer_signal", "peer_wait"):

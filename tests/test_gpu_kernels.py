@@ -584,6 +584,23 @@ def test_rmsnorm(K, rows, d, heads):
     _check_status()
 
 
+@pytest.mark.parametrize("B,S,H,Hk", [(1, 1, 1, 1), (2, 33, 4, 1), (1, 300, 8, 2), (3, 64, 5, 5)])
+def test_rope_pair_is_two_ropes(K, B, S, H, Hk):
+    """One launch for q and k, here column slices of one buffer, gives bit for bit what two launches give."""
+    torch.manual_seed(S)
+    both = torch.randn(B, S, H + Hk, 128, device="cuda", dtype=torch.bfloat16)
+    q, k = both[:, :, :H], both[:, :, H:]
+    cos, sin = ref.rope_tables(S, 128, 10000.0, device="cuda")
+    for sign in (1.0, -1.0):
+        got = torch.zeros(B, S, H, 128, device="cuda", dtype=torch.bfloat16), torch.zeros_like(k, memory_format=torch.contiguous_format)
+        want = torch.zeros_like(got[0]), torch.zeros_like(got[1])
+        K.rope_pair(q, k, *got, cos, sin, sign=sign)
+        K.rope(q, want[0], cos, sin, sign=sign)
+        K.rope(k, want[1], cos, sin, sign=sign)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    _check_status()
+
+
 def test_rope_and_glu(K):
     dev = "cuda"
     torch.manual_seed(5)
