@@ -45,9 +45,9 @@ constexpr int TMEM_COLS = 512;
 constexpr int S_COL = 0;      // S of tile i: columns [128 i, 128 i + 128); P (bf16x2, 64 cols) over its first 64
 constexpr int O_COL = 256;    // O of tile i: columns [256 + 128 i, ...)
 constexpr int GROUP = 8;      // (batch, head) slices per scheduling group
-constexpr int N_SCHED = 64;   // ring of work counters (one per launch in flight)
+constexpr int N_SCHED = 64;   // ring of (work counter, CTAs done) pairs, one per launch in flight
 
-__device__ int g_sched[N_SCHED];
+__device__ int g_sched[2 * N_SCHED];
 
 struct Params {
   int B, S, H, Hkv;
@@ -61,7 +61,7 @@ struct Params {
   long long o_sb, o_ss, o_sh;  // element strides of O
   float* lse;                  // [B, H, S]
   int* status;
-  int* sched;                  // work counter, zero at launch
+  int* sched;                  // work counter and number of CTAs done; both zero between launches
   int n_pairs, n_items;        // query-tile pairs per (batch, head); items in the padded schedule
 };
 
@@ -572,6 +572,15 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  // The last CTA clears the pair for the launch that takes it next (a memset before every launch cost the host about 5 us
+  // and the stream 1.3).  Every CTA comes here, also after a wait that gave up.
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(p.sched + 1, 1) == (int)gridDim.x - 1) {
+      p.sched[0] = 0;
+      p.sched[1] = 0;
+    }
+  }
 }
 
 }  // namespace fa_fwd
@@ -627,7 +636,7 @@ extern "C" int ob_flash_attn_fwd(const ObAttnArgs* a, cudaStream_t stream) {
     attr_set[dev] = true;
   }
   // persistent CTAs, one per SM, fed from a work counter: a ring of counters so that launches in flight on different
-  // streams never share one; the launch's counter is cleared in stream order just before the kernel
+  // streams never share one; each launch leaves its counter cleared
   static int n_sm[64] = {};
   static int* sched_base[64] = {};
   if (n_sm[dev] == 0) {
@@ -639,11 +648,10 @@ extern "C" int ob_flash_attn_fwd(const ObAttnArgs* a, cudaStream_t stream) {
     n_sm[dev] = n;
   }
   static std::atomic<unsigned> launch_no{0};
-  p.sched = sched_base[dev] + launch_no.fetch_add(1) % fa_fwd::N_SCHED;
+  p.sched = sched_base[dev] + 2 * (launch_no.fetch_add(1) % fa_fwd::N_SCHED);
   p.n_pairs = (a->S + 2 * fa_fwd::TQ - 1) / (2 * fa_fwd::TQ);
   const int groups = (a->B * a->H + fa_fwd::GROUP - 1) / fa_fwd::GROUP;
   p.n_items = groups * fa_fwd::GROUP * p.n_pairs;
-  OB_CUDA_OK(cudaMemsetAsync(p.sched, 0, sizeof(int), stream));
   const int valid_items = a->B * a->H * p.n_pairs;
   dim3 grid(valid_items < n_sm[dev] ? valid_items : n_sm[dev]);
   fa_fwd::flash_fwd_kernel<<<grid, fa_fwd::THREADS, fa_fwd::SMEM_BYTES, stream>>>(tq, tk, tv, p);
