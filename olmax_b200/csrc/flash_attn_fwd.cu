@@ -382,6 +382,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t t_s = t_lane + S_COL + (uint32_t)tile * 128u;
     const uint32_t t_o = t_lane + O_COL + (uint32_t)tile * 128u;
     const bool capped = p.softcap > 0.f;
+    const float2 over_cap2 = make_float2(p.scale_over_cap, p.scale_over_cap), cap2 = make_float2(p.cap_log2, p.cap_log2);
     const float sc = capped ? 1.0f : p.scale_log2;   // soft-capped scores are already in the log2 domain
     bool ok = true;
     uint32_t n_item = 0, cs = 0, ce = 0;
@@ -451,8 +452,12 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-              for (int i = 0; i < 32; ++i)
-                r[c][i] = __float_as_uint(p.cap_log2 * fast_tanh(__uint_as_float(r[c][i]) * p.scale_over_cap));
+              for (int i = 0; i < 32; i += 2) {
+                const float2 x = mul2(make_float2(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), over_cap2);
+                const float2 t = mul2(make_float2(fast_tanh(x.x), fast_tanh(x.y)), cap2);
+                r[c][i] = __float_as_uint(t.x);
+                r[c][i + 1] = __float_as_uint(t.y);
+              }
           }
           if (need_mask) {
 #pragma unroll
