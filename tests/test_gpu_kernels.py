@@ -374,8 +374,10 @@ def test_flash_attention(K, B, S, H, Hkv, causal, window, softcap):
     (2, 257, 3, 3, True, 64, 0.0),        # window narrower than a tile: both diagonal edges cut the same tile
     (1, 300, 2, 2, True, 130, 25.0),      # window just wider than a tile, with the soft-cap
     (1, 127, 8, 2, False, -1, 0.0),       # no mask but the sequence's end
-    (4, 640, 16, 8, True, -1, 0.0),       # more key tiles than one scheduling group holds: 160 CTAs, LPT order
-    (2, 1300, 64, 32, True, -1, 0.0),     # 704 CTAs: groups of eight slices
+    (4, 640, 16, 8, True, -1, 0.0),       # 160 items, longest first; twelve CTAs take two
+    (2, 1300, 64, 32, True, -1, 0.0),     # 704 work items: groups of eight slices, several items per CTA
+    (2, 1100, 24, 12, True, 200, 0.0),    # 216 items with a window: some CTAs take a second item, loops of one to six tiles
+    (2, 1100, 24, 12, True, 200, 30.0),   # the same with the soft-cap: one CTA per item
 ])
 def test_flash_attention_backward_tile_edges(K, B, S, H, Hkv, causal, window, softcap):
     """Gradients against fp32 autograd where tiles are cut.  Tolerance: dS, P, the inputs and the result are each rounded
