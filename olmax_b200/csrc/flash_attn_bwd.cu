@@ -9,7 +9,8 @@
 //
 // Roles (16 warps): two compute warpgroups form P and dS (thread <-> key row, 64 query columns), one warpgroup drains the
 // dQ partial to an fp32 scratch tensor with TMA reduce-adds from a staging buffer of its own, and one warpgroup holds
-// the TMA warp, the MMA warp and the warp that brings the row statistics into shared memory.  The TMA warp also hands out the work items.
+// the TMA warp, which also hands out the work items, the MMA warp and the warp that brings the row statistics into shared
+// memory.
 //
 // The MMA order is dV(j), S(j+1) | dQ(j), dK(j), dP(j+1): S(j+1) is issued while the compute warps form dS(j), so that
 // P(j+1) is formed under dQ(j) and dK(j); dQ(j) is drained under dK(j); and dS(j+1) is formed under dV(j+1), S(j+2).
@@ -17,9 +18,9 @@
 // 128 B/clk), and with the staging of dQ and the loads about 512 KB pass the port per tile pair (4100 cycles, against
 // 2560 cycles of tensor work and about 1024 cycles of MUFU work for the exponentials).
 //
-// Forward + backward through the attention op, before (P and dS through shared memory, dQ drained by the compute warps,
-// every MMA waiting for the previous stage of the same tile) and now: B 2, S 4096, H 32 causal 1427 -> 1239 us; B 3,
-// S 1515, H 40 / 8 582 -> 424 us; B 1, S 8192, H 32 / 16, window 4096, soft-cap 2465 -> 1892 us.
+// All kernels of the backward, before (P and dS through shared memory, dQ drained by the compute warps, every MMA waiting for
+// the previous stage of the same tile) and now: B 2, S 4096, H 32 causal 1058 -> 723 us; B 3, S 1515, H 40 / 8 464 -> 238 us;
+// B 1, S 8192, H 32 / 16, window 4096, soft-cap 1858 -> 1080 us.
 //
 // The math is the standard recompute form: P = exp(S - lse), dS = P * (dP - delta) with the softmax scale applied to the
 // sums dQ and dK, delta = rowsum(dO * O) from a pre-pass; a tanh soft-cap multiplies dS by (1 - tanh^2).
