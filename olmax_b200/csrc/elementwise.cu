@@ -11,6 +11,7 @@
 #include <limits.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "host_common.h"
 #include "sm100.cuh"
@@ -160,9 +161,12 @@ __global__ void __launch_bounds__(NORM_THREADS)
 }
 
 // dx = rstd * (w*dy - xhat * mean(w*dy*xhat)) (+ dsum);  dw += sum_rows dy * xhat  (fp32 atomics, accumulating)
-// (next row group fetched before the current one is reduced, as in the forward kernel)
-template <int TPR, int VPT>
-__global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2))
+// (Next row group fetched before the current one is reduced, as in the forward kernel.  DSUM, with a residual gradient: that
+// row too; read after the row's barriers it cost [65536, 1024] 127 us against 111, [5560, 5120] 70 against 59.  The rows in
+// flight then need the registers of one block per SM: [8192, 4096] 64 -> 57 us, 67 with the limit of the plain form, which
+// in turn would lose 45 -> 51 us with this one's.)
+template <int TPR, int VPT, bool DSUM>
+__global__ void __launch_bounds__(NORM_THREADS, DSUM ? (VPT <= 1 ? 3 : 2) : (VPT <= 1 ? 4 : VPT <= 2 ? 3 : 2))
     rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                        const float* __restrict__ rstd_in, const bf16* __restrict__ dsum, bf16* __restrict__ dx,
                        float* __restrict__ dw, long long rows, int d, int heads, long long ld_dy, long long ld_x,
@@ -178,12 +182,13 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
   for (int i = 0; i < VPT; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-  bf16x8 ng[VPT], nx[VPT];
+  bf16x8 ng[VPT], nx[VPT], nd[VPT];
   float nrstd = 0.f;
   auto fetch = [&](long long row0) {
     const long long row = row0 + sub;
     if (row < rows) {
       const long long ody = row_offset(row, heads, ld_dy, d), ox = row_offset(row, heads, ld_x, d);
+      [[maybe_unused]] const long long odx = row_offset(row, heads, ld_dx, d);
       nrstd = rstd_in[row];
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
@@ -191,6 +196,7 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
         if (vi < nvec) {
           ng[i] = load_raw8(dy + ody + vi * 8);
           nx[i] = load_raw8(x + ox + vi * 8);
+          if constexpr (DSUM) nd[i] = load_raw8(dsum + odx + vi * 8);
         }
       }
     }
@@ -203,6 +209,7 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
     const long long odx = live ? row_offset(row, heads, ld_dx, d) : 0;
     const float rstd = live ? nrstd : 0.f;
     float g[VPT][8], xh[VPT][8];
+    bf16x8 cd[VPT];   // this row's dsum, raw (the fetch below overwrites nd)
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -211,6 +218,7 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
         float wv[8];
         unpack8(ng[i], g[i]);
         unpack8(nx[i], xh[i]);
+        if constexpr (DSUM) cd[i] = nd[i];
         load8(w + vi * 8, wv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -230,9 +238,9 @@ __global__ void __launch_bounds__(NORM_THREADS, VPT <= 1 ? 4 : (VPT <= 2 ? 3 : 2
         float o[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = rstd * (g[i][j] - xh[i][j] * dot);
-        if (dsum != nullptr) {
+        if constexpr (DSUM) {
           float e[8];
-          load8(dsum + odx + vi * 8, e);
+          unpack8(cd[i], e);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += e[j];
         }
@@ -845,10 +853,14 @@ extern "C" int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   return norm_dispatch(d, "rmsnorm", [&](auto shape) {
     using S = decltype(shape);
     const int rpb = NORM_THREADS / S::TPR;
-    constexpr auto kernel = rmsnorm_bwd_kernel<S::TPR, S::VPT>;
-    kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
-        (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dsum, (bf16*)dx, dw, rows, d, heads, ld_dy,
-        ld_x, ld_dx, dw_scale);
+    auto run = [&](auto with_dsum) {
+      constexpr auto kernel = rmsnorm_bwd_kernel<S::TPR, S::VPT, decltype(with_dsum)::value>;
+      kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
+          (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dsum, (bf16*)dx, dw, rows, d, heads, ld_dy,
+          ld_x, ld_dx, dw_scale);
+    };
+    if (dsum != nullptr) run(std::true_type{});
+    else run(std::false_type{});
   });
 }
 
