@@ -48,6 +48,45 @@ def test_linear_value_and_grad(bias):
         assert torch.allclose(g["bias"], p["bias"].grad, atol=1e-5)
 
 
+class _Doubled(Linear):
+    def forward(self, x):
+        return 2 * super().forward(x)
+
+
+class _Unrotated(RotaryPositionalEmbedding):
+    def forward(self, x, *args, **kw):
+        return x
+
+
+@pytest.mark.parametrize("how", ["hook", "pre-hook", "subclass", "attribute"])
+@pytest.mark.parametrize("name", ["q_proj", "k_proj", "v_proj", "rope"])
+def test_attention_projections_and_rotation_that_a_user_has_changed(name, how):
+    """Projections and rotations of one block may run as one call: what was hooked, subclassed or replaced still runs."""
+    cfg = MultiheadSelfAttentionConfig(n_heads=2, n_kv_heads=2, head_dim=16, rope=RotaryPositionalEmbeddingConfig())
+    attn = _build(lambda: cfg.build(24))
+    x = torch.randn(6, 24)
+    plain = attn._qkv(x, 1, None)
+    mod = getattr(attn, name)
+    if how == "hook":
+        mod.register_forward_hook(lambda m, args, y: args[0] if name == "rope" else 2 * y)
+    elif how == "pre-hook":
+        mod.register_forward_pre_hook(lambda m, args: (2 * args[0], *args[1:]))
+    elif how == "subclass":
+        mod.__class__ = _Unrotated if name == "rope" else _Doubled
+    else:
+        forward = mod.forward
+        mod.forward = lambda t, *args, **kw: 2 * forward(t, *args, **kw)
+    got = attn._qkv(x, 1, None)
+    for key, g, w in zip("qkv", got, plain):
+        if name == "rope" and key != "v":
+            want = 2 * w
+            if how in ("hook", "subclass"):
+                want = getattr(attn, key + "_proj")(x).view(1, 6, 2, 16)
+        else:
+            want = 2 * w if name[0] == key else w
+        assert torch.allclose(g, want, atol=1e-6), key
+
+
 @pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
 def test_gated_mlp_value_and_grad(act):
     mlp = _build(lambda: GatedMLP(16, 40, activation=act))
