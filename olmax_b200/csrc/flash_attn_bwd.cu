@@ -26,9 +26,6 @@
 // sums dQ and dK, delta = rowsum(dO * O) from a pre-pass; a tanh soft-cap multiplies dS by (1 - tanh^2).
 //
 // Counterpart of the autodiff of `olmax/nn/attention.py:96-103` (cuDNN backward in the reference).
-#include <algorithm>
-#include <atomic>
-
 #include "flash_attn.h"
 #include "flash_attn_noalloc.h"
 #include "host_common.h"
@@ -63,18 +60,13 @@ constexpr int COMPUTE_WARPS = 8;
 // registers per thread after the split; 2 * 168 + 88 + 88 = 512 = 4 * the 128 of the launch
 constexpr int REGS_COMPUTE = 168, REGS_DRAIN = 88, REGS_ISSUE = 88;
 constexpr int TMEM_COLS = 512;
-constexpr int N_SCHED = 64;   // ring of work counters (one per launch in flight)
 constexpr int C_S = 0, C_DP = 128, C_DK = 256, C_DV = 384;
-
-__device__ int g_sched[N_SCHED];
 
 struct Params {
   int B, S, H, Hkv;
   int Sk, q_off;   // key length; key-axis position of query row 0
   int causal, window;
   int kv_tiles, group;   // key tiles per slice; (batch, kv-head) slices per scheduling group
-  int n_items;           // key tiles in all
-  int* sched;            // next work item beyond the CTAs' first ones (set to the grid by the pre-pass)
   float scale, scale_log2, softcap, scale_over_cap, cap_log2;
   const float* lse;
   const float* delta;
@@ -128,11 +120,12 @@ __device__ __forceinline__ Item decode_item(const Params& p, int w) {
 }
 
 // CAPPED: with a soft-cap.  Its code and registers stay out of the plain kernel, and the other way round.
-// PERSISTENT: one CTA per SM takes work items from a counter, so that the next item's loads, first scores and dP run under the
-// write-out of dK / dV; else one CTA per item.  Without a soft-cap the three kernels of the backward gain by it: B 64, S 1024,
-// H 8 682 -> 618 us (4.5 query tiles per item), B 2, S 4096, H 32 748 -> 723, B 3, S 1515, H 40 / 8 and B 1, S 8192, H 32 / 16,
-// window 4096 unchanged.  With one, the compute warps bound the loop and the longer-lived state costs them: B 1, S 8192,
-// H 32 / 16 1364 -> 1438 us, with window 4096 1058 -> 1075; so the capped kernel keeps one CTA per item.
+// PERSISTENT: the CTA that runs on an SM takes over the items of CTAs that have not started, so that the next item's loads,
+// first scores and dP run under the write-out of dK / dV; else every CTA has its one item.  Without a soft-cap the three
+// kernels of the backward gain by it: B 64, S 1024, H 8 682 -> 618 us (4.5 query tiles per item), B 2, S 4096, H 32
+// 748 -> 723, B 3, S 1515, H 40 / 8 and B 1, S 8192, H 32 / 16, window 4096 unchanged.  With one, the compute warps bound
+// the loop and the longer-lived state costs them: B 1, S 8192, H 32 / 16 1364 -> 1438 us, with window 4096 1058 -> 1075;
+// so the capped kernel keeps one item per CTA.
 template <bool CAPPED>
 __global__ void __launch_bounds__(THREADS, 1)
     flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -161,6 +154,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* item_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [2] work item, < 0: end
+  uint64_t* taken_full = bars + 26;
+  uint4* taken = reinterpret_cast<uint4*>(bars + 28);   // the scheduler's last answer, see next_cta_request
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -197,6 +192,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_init(&item_full[s], 1);
       mbar_init(&item_empty[s], 2 + 4 + COMPUTE_WARPS);
     }
+    mbar_init(taken_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
     fence_proxy_async();
@@ -245,10 +241,12 @@ __global__ void __launch_bounds__(THREADS, 1)
           // not before the last dV of the current item: a CTA that still has work would take an item from one that has none
           if (g > 0) dead = !mbar_wait(do_empty, (g & 1u) ^ 1u, abort_flag, p.status, 691);
           if (dead) break;
-          if (lane == 0) w = atomicAdd(p.sched, 1);
-          w = __shfl_sync(0xffffffffu, w, 0);
-          if (w >= p.n_items) w = -1;
           const uint32_t k = n_item - 1;
+          if (lane == 0) next_cta_request(taken, taken_full);
+          dead = !mbar_wait(taken_full, k & 1u, abort_flag, p.status, 692);
+          if (dead) break;
+          w = next_cta_answer(taken);
+          __syncwarp();
           dead = !mbar_wait(&item_empty[k & 1], ((k >> 1) & 1u) ^ 1u, abort_flag, p.status, 690);
           if (dead) break;
           if (lane == 0) {
@@ -736,9 +734,7 @@ __device__ __forceinline__ void row_coords(unsigned row, int S, int H, int& b, i
 __global__ void __launch_bounds__(ROW_THREADS)
     attn_delta_kernel(const bf16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
                       const bf16* __restrict__ d_o, long long do_sb, long long do_ss, long long do_sh,
-                      float* __restrict__ delta, float* __restrict__ dq_acc, int S, int H, unsigned rows, bool wide_o,
-                      int* __restrict__ sched, int main_grid) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *sched = main_grid;   // the main kernel's work counter
+                      float* __restrict__ delta, float* __restrict__ dq_acc, int S, int H, unsigned rows, bool wide_o) {
   const int l16 = threadIdx.x & 15;
   const unsigned row0 = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 4);
   int b[ROWS_PT], s[ROWS_PT], h[ROWS_PT];
@@ -858,25 +854,11 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   const int kv_tiles = (Sk + 127) / 128;
   const long long slices = (long long)a->B * a->Hkv, items = slices * kv_tiles;
   if (items > 0x7fffffffLL) OB_FAIL(-4, "%lld key tiles exceed the grid", items);
-  // work counters: a ring, so that launches in flight on different streams never share one
-  static int* sched_base[64] = {};
-  static int n_sm[64] = {};
-  if (n_sm[dev] == 0) {
-    int n = 0;
-    OB_CUDA_OK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    void* sym = nullptr;
-    OB_CUDA_OK(cudaGetSymbolAddress(&sym, fa_bwd::g_sched));
-    sched_base[dev] = static_cast<int*>(sym);
-    n_sm[dev] = n;
-  }
-  static std::atomic<unsigned> launch_no{0};
-  int* sched = sched_base[dev] + launch_no.fetch_add(1) % fa_bwd::N_SCHED;
-  const unsigned grid = (unsigned)(a->softcap > 0.f ? items : std::min<long long>(items, n_sm[dev]));
   const unsigned nblk = (unsigned)((rows + fa_bwd::ROWS_PER_BLOCK - 1) / fa_bwd::ROWS_PER_BLOCK);
   fa_bwd::attn_delta_kernel<<<nblk, fa_bwd::ROW_THREADS, 0, stream>>>(
       reinterpret_cast<const bf16*>(a->o), a->o_sb, a->o_ss, a->o_sh, reinterpret_cast<const bf16*>(a->d_o), a->do_sb,
       a->do_ss, a->do_sh, delta, dq_accum, a->S, a->H, (unsigned)rows,
-      fa_bwd::wide_rows(a->o, a->o_sb, a->o_ss, a->o_sh), sched, (int)grid);
+      fa_bwd::wide_rows(a->o, a->o_sb, a->o_ss, a->o_sh));
   OB_CUDA_OK(cudaGetLastError());
 
   fa_bwd::Params p;
@@ -898,10 +880,8 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   // Few items per SM: the longest loops of all slices first, or the last ones to start set the time.  Many: groups of eight
   // slices, whose Q / dO / dQ (8 MB per 1024 rows, times the heads per kv-head) stay in L2 while their key tiles run.
   p.group = items <= 4 * 148 ? (int)slices : 8;
-  p.n_items = (int)items;
-  p.sched = sched;
   const auto kernel = a->softcap > 0.f ? fa_bwd::flash_bwd_kernel<true> : fa_bwd::flash_bwd_kernel<false>;
-  kernel<<<grid, fa_bwd::THREADS, fa_bwd::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdq, p);
+  kernel<<<(unsigned)items, fa_bwd::THREADS, fa_bwd::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdq, p);
   OB_CUDA_OK(cudaGetLastError());
   fa_bwd::attn_dq_convert_kernel<<<nblk, fa_bwd::ROW_THREADS, 0, stream>>>(
       dq_accum, reinterpret_cast<bf16*>(a->dq), a->dq_sb, a->dq_ss, a->dq_sh, a->scale, a->S, a->H, (unsigned)rows,

@@ -103,6 +103,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 }
 
 // ---------------------------------------------------------------------------------------------------
+// Work items from the launch itself: a grid has one CTA per item, and a running CTA takes the index of one that has not
+// started, which then never does.  Nothing in global memory is kept for it, so launches share no state whatever streams,
+// threads or captured graphs they come from.  One thread asks (and reads the last answer before it asks again: the answer
+// is written by the async proxy); after an answer that there is none it may not ask again.
+// ---------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void next_cta_request(uint4* answer, uint64_t* bar) {
+  fence_proxy_async();   // the last answer has been read
+  mbar_arrive_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// Once the barrier's phase is through: blockIdx.x of the CTA taken, -1: all have started.
+__device__ __forceinline__ int next_cta_answer(const uint4* answer) {
+  unsigned long long lo, hi;
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(smem_u32(answer)) : "memory");
+  int x = -1;
+  asm volatile(
+      "{\n"
+      ".reg .b128 r;\n"
+      ".reg .pred p;\n"
+      "mov.b128 r, {%1, %2};\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n"
+      "}\n"
+      : "+r"(x)
+      : "l"(lo), "l"(hi));
+  return x;
+}
+
+// ---------------------------------------------------------------------------------------------------
 // TMA (tile mode, local global memory only, never multicast)
 // ---------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {

@@ -414,6 +414,48 @@ def test_flash_attention_backward_with_rows_of_8_byte_alignment(K, B, S, H):
     _check_status()
 
 
+def _beside_each_other(small, large, n):
+    """What ``n`` calls of each give when two streams run them side by side without waiting for the host, and again with
+    ``large`` captured in a graph and replayed beside the calls of ``small``: ``[(expected by, results), ...]``."""
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    out = [[], []]
+    torch.cuda.synchronize()
+    for _ in range(n):
+        for i, (s, fn) in enumerate(((s1, small), (s2, large))):
+            with torch.cuda.stream(s):
+                out[i].append(fn())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s2):
+        captured = large()
+    for _ in range(n):
+        with torch.cuda.stream(s1):
+            out[0].append(small())
+        with torch.cuda.stream(s2):
+            graph.replay()
+            out[1].append(tuple(t.clone() for t in captured))
+    torch.cuda.synchronize()
+    return out
+
+
+def test_flash_attention_backward_calls_beside_each_other(K):
+    """More backward launches in flight on two streams, and in a replayed graph, than any ring of shared counters would
+    hold: every call gives the gradients of a call on its own (dK and dV to the bit; dQ's fp32 sums meet in any order)."""
+    torch.manual_seed(29)
+    calls, want = [], []
+    for B, S, H, Hkv in ((1, 200, 2, 2), (2, 1024, 8, 4)):
+        q, d_o = (torch.randn(B, S, H, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        k, v = (torch.randn(B, S, Hkv, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        args = (q, k, v, *K.flash_attn_fwd(q, k, v), d_o)
+        calls.append(lambda args=args: K.flash_attn_bwd(*args))
+        want.append(calls[-1]())
+    for results, (dq, dk, dv) in zip(_beside_each_other(*calls, 80), want):
+        for got in results:
+            assert rel_err(got[0], dq.float()) < 2e-3
+            assert torch.equal(got[1], dk) and torch.equal(got[2], dv)
+    _check_status()
+
+
 @pytest.mark.parametrize("S,Sk,q_off,window,softcap", [
     (256, 512, 256, -1, 0.0),      # late query chunk against the causally visible prefix
     (128, 128, 384, -1, 0.0),      # ring block far below the diagonal: every key visible
