@@ -1,11 +1,11 @@
 // Flash-attention forward for sm_100a (head_dim 128, bf16 in/out, fp32 softmax statistics).
 //
-// A persistent CTA (one per SM) takes work items from a counter in global memory.  A work item is a pair of
-// 128-row query tiles of one (batch, head).  S = Q K^T and O += P V run on tcgen05 tensor cores with accumulators in
-// TMEM: each query tile owns 128 fp32 columns for S and 128 for O (512 columns in all); P (bf16) is written back
-// over its S columns and is consumed from TMEM as the A operand of the second MMA, so P never touches shared
-// memory.  Each query tile has its own softmax warpgroup (4 warps, one thread per query row, the whole 128-score
-// row in registers, so no exchange between threads), and the MMA warp interleaves the two tiles:
+// A work item is a pair of 128-row query tiles of one (batch, head).  The grid has one CTA per item; the CTA that runs on
+// an SM takes over the items of CTAs that have not started, one after the other.  S = Q K^T and O += P V run on tcgen05
+// tensor cores with accumulators in TMEM: each query tile owns 128 fp32 columns for S and 128 for O (512 columns in
+// all); P (bf16) is written back over its S columns and is consumed from TMEM as the A operand of the second MMA, so P
+// never touches shared memory.  Each query tile has its own softmax warpgroup (4 warps, one thread per query row, the
+// whole 128-score row in registers, so no exchange between threads), and the MMA warp interleaves the two tiles:
 //     P V (tile 0, keys j), Q K^T (tile 0, keys j+1), P V (tile 1, keys j), Q K^T (tile 1, keys j+1), ...
 // so that the tensor cores work on one tile while the other tile is in its softmax.  P is announced in two halves, so
 // that P V of the first 64 keys runs under the exponentials of the rest.  K and V tiles go through rings shared by
@@ -23,8 +23,6 @@
 //
 // Takes the place of the cuDNN / TransformerEngine fused attention the reference calls in
 // `olmax/nn/attention.py:52-109`; soft-cap has no counterpart there.
-#include <atomic>
-
 #include "flash_attn.h"
 #include "host_common.h"
 #include "sm100.cuh"
@@ -45,9 +43,6 @@ constexpr int TMEM_COLS = 512;
 constexpr int S_COL = 0;      // S of tile i: columns [128 i, 128 i + 128); P (bf16x2, 64 cols) over its first 64
 constexpr int O_COL = 256;    // O of tile i: columns [256 + 128 i, ...)
 constexpr int GROUP = 8;      // (batch, head) slices per scheduling group
-constexpr int N_SCHED = 64;   // ring of (work counter, CTAs done) pairs, one per launch in flight
-
-__device__ int g_sched[2 * N_SCHED];
 
 struct Params {
   int B, S, H, Hkv;
@@ -61,8 +56,7 @@ struct Params {
   long long o_sb, o_ss, o_sh;  // element strides of O
   float* lse;                  // [B, H, S]
   int* status;
-  int* sched;                  // work counter and number of CTAs done; both zero between launches
-  int n_pairs, n_items;        // query-tile pairs per (batch, head); items in the padded schedule
+  int n_pairs;                 // query-tile pairs per (batch, head)
 };
 
 __device__ __forceinline__ float fast_tanh(float x) {
@@ -117,16 +111,15 @@ __device__ __forceinline__ Geo item_geometry(const Params& p, int pair, int h, i
   return g;
 }
 
-// schedule position -> (pair, h, b); false for the padding of the last group
-__device__ __forceinline__ bool decode_item(const Params& p, int w, int& pair, int& h, int& b) {
+// schedule position -> (pair, h, b)
+__device__ __forceinline__ void decode_item(const Params& p, int w, int& pair, int& h, int& b) {
   const int per_group = GROUP * p.n_pairs;
   const int g = w / per_group, r = w - g * per_group;
-  pair = p.n_pairs - 1 - r / GROUP;          // heaviest (longest causal rows) first
-  const int bh = g * GROUP + r % GROUP;
-  if (bh >= p.B * p.H) return false;
+  const int slices = min(GROUP, p.B * p.H - g * GROUP);   // the last group may have fewer
+  pair = p.n_pairs - 1 - r / slices;          // heaviest (longest causal rows) first
+  const int bh = g * GROUP + r % slices;
   b = bh / p.H;
   h = bh - b * p.H;
-  return true;
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -153,6 +146,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* item_slot = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [2][4]: pair (< 0: end), h, b
+  uint64_t* taken_full = bars + 36;
+  uint4* taken = reinterpret_cast<uint4*>(bars + 38);   // the scheduler's last answer, see next_cta_request
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -169,6 +164,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
+    mbar_init(taken_full, 1);
     for (int i = 0; i < STK; ++i) {
       mbar_init(k_full + i, 1);
       mbar_init(k_empty + i, 1);
@@ -203,15 +199,17 @@ __global__ void __launch_bounds__(THREADS, 1)
       tma_prefetch_desc(&tmV);
     }
     uint32_t n_item = 0, k_it = 0;
+    bool asked = false;   // for the next item, answer not yet read
     while (!dead) {
-      int pair = -1, h = 0, b = 0;
-      for (;;) {
-        int w = 0;
-        if (lane == 0) w = atomicAdd(p.sched, 1);
-        w = __shfl_sync(0xffffffffu, w, 0);
-        if (w >= p.n_items) { pair = -1; break; }
-        if (decode_item(p, w, pair, h, b)) break;
+      int w = (int)blockIdx.x, pair = -1, h = 0, b = 0;
+      if (n_item > 0) {
+        dead = !mbar_wait(taken_full, (n_item & 1u) ^ 1u, abort_flag, p.status, 404);
+        if (dead) break;
+        w = next_cta_answer(taken);
+        asked = false;
+        __syncwarp();
       }
+      if (w >= 0) decode_item(p, w, pair, h, b);
       const uint32_t slot = n_item & 1u;
       dead = !mbar_wait(item_empty + slot, ((n_item >> 1) & 1u) ^ 1u, abort_flag, p.status, 400);
       if (dead) break;
@@ -246,6 +244,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int u = g.ulo; u <= g.uhi; ++u, ++k_it) {
         if (u < g.uhi) load_k(u + 1, k_it + 1);
         const uint32_t st = k_it % STV, ph = (k_it / STV) & 1u;
+        // the next item, as late as its answer still comes in time: a CTA that has work left takes none from one that has not
+        if (u == g.uhi && !dead) {
+          if (lane == 0) next_cta_request(taken, taken_full);
+          asked = true;
+        }
         if (!dead) dead = !mbar_wait(v_empty + st, ph ^ 1u, abort_flag, p.status, 403);
         if (leader && !dead) {
           mbar_arrive_expect_tx(v_full + st, TILE_BYTES);
@@ -255,6 +258,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       ++n_item;
     }
+    // (after a wait that gave up: the answer must not arrive in another CTA's shared memory)
+    if (asked) mbar_wait(taken_full, (n_item & 1u) ^ 1u, abort_flag, p.status, 405);
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -577,15 +582,6 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
-  // The last CTA clears the pair for the launch that takes it next (a memset before every launch cost the host about 5 us
-  // and the stream 1.3).  Every CTA comes here, also after a wait that gave up.
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(p.sched + 1, 1) == (int)gridDim.x - 1) {
-      p.sched[0] = 0;
-      p.sched[1] = 0;
-    }
-  }
 }
 
 }  // namespace fa_fwd
@@ -640,26 +636,10 @@ extern "C" int ob_flash_attn_fwd(const ObAttnArgs* a, cudaStream_t stream) {
                                     fa_fwd::SMEM_BYTES));
     attr_set[dev] = true;
   }
-  // persistent CTAs, one per SM, fed from a work counter: a ring of counters so that launches in flight on different
-  // streams never share one; each launch leaves its counter cleared
-  static int n_sm[64] = {};
-  static int* sched_base[64] = {};
-  if (n_sm[dev] == 0) {
-    int n = 0;
-    OB_CUDA_OK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    void* sym = nullptr;
-    OB_CUDA_OK(cudaGetSymbolAddress(&sym, fa_fwd::g_sched));
-    sched_base[dev] = static_cast<int*>(sym);
-    n_sm[dev] = n;
-  }
-  static std::atomic<unsigned> launch_no{0};
-  p.sched = sched_base[dev] + 2 * (launch_no.fetch_add(1) % fa_fwd::N_SCHED);
   p.n_pairs = (a->S + 2 * fa_fwd::TQ - 1) / (2 * fa_fwd::TQ);
-  const int groups = (a->B * a->H + fa_fwd::GROUP - 1) / fa_fwd::GROUP;
-  p.n_items = groups * fa_fwd::GROUP * p.n_pairs;
-  const int valid_items = a->B * a->H * p.n_pairs;
-  dim3 grid(valid_items < n_sm[dev] ? valid_items : n_sm[dev]);
-  fa_fwd::flash_fwd_kernel<<<grid, fa_fwd::THREADS, fa_fwd::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  const long long items = (long long)a->B * a->H * p.n_pairs;
+  if (items > 0x7fffffffLL) OB_FAIL(-4, "%lld query-tile pairs exceed the grid", items);
+  fa_fwd::flash_fwd_kernel<<<(unsigned)items, fa_fwd::THREADS, fa_fwd::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   OB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -438,6 +438,26 @@ def _beside_each_other(small, large, n):
     return out
 
 
+def test_flash_attention_forward_calls_beside_each_other(K):
+    """The same for the forward, with grids of different sizes and a last group of fewer than eight slices: results to the
+    bit.  A launch on its own afterwards is right too: nothing is left behind."""
+    torch.manual_seed(28)
+    calls, want = [], []
+    for B, S, H, Hkv in ((1, 200, 3, 3), (3, 1024, 4, 2)):
+        q = torch.randn(B, S, H, 128, device="cuda", dtype=torch.bfloat16)
+        k, v = (torch.randn(B, S, Hkv, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        calls.append(lambda args=(q, k, v): K.flash_attn_fwd(*args))
+        want.append(calls[-1]())
+        o, lse = ref.attention(q.float(), k.float(), v.float(), True, -1, 0.0)
+        assert rel_err(want[-1][0], o) < 6e-3 and rel_err(want[-1][1], lse) < 1e-3
+    results = _beside_each_other(*calls, 80)
+    for _ in range(65):
+        results[1].append(calls[1]())
+    for got, (o, lse) in zip(results, want):
+        assert all(torch.equal(g[0], o) and torch.equal(g[1], lse) for g in got)
+    _check_status()
+
+
 def test_flash_attention_backward_calls_beside_each_other(K):
     """More backward launches in flight on two streams, and in a replayed graph, than any ring of shared counters would
     hold: every call gives the gradients of a call on its own (dK and dV to the bit; dQ's fp32 sums meet in any order)."""
