@@ -806,6 +806,15 @@ static inline int resident_grid(long long work_blocks, size_t smem) {
   return (int)(work_blocks < cap ? (work_blocks < 1 ? 1 : work_blocks) : cap);
 }
 
+// More than 48 KB of shared memory, the kernel's static `red` counted in, need the opt-in (a per-device attribute): always
+// for the layout's longest row, so that no thread lowers it between another's opt-in and launch.  An error is left for the
+// check after the launch.
+template <auto KERNEL>
+static inline void allow_smem(size_t smem, size_t longest) {
+  if (smem + NORM_THREADS / 32 * sizeof(float) > 48 * 1024)
+    cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)longest);
+}
+
 // Thread layout of the normalisation kernels for a row of d elements: TPR threads share a row and each keeps VPT
 // 8-element vectors of it in registers.  Instantiating the smallest VPT that covers d keeps the register count (and
 // with it the number of resident blocks, i.e. the bytes in flight) right for the common widths.
@@ -885,9 +894,8 @@ extern "C" int ob_layernorm_bwd(const void* dy, const void* x, const void* w, co
   return norm_dispatch(d, "layernorm", [&](auto shape) {
     using S = decltype(shape);
     const int rpb = NORM_THREADS / S::TPR;
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(layernorm_bwd_kernel<S::TPR, S::VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     constexpr auto kernel = layernorm_bwd_kernel<S::TPR, S::VPT>;
+    allow_smem<kernel>(smem, S::TPR * S::VPT * 8 * 2 * sizeof(float));
     kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
         (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd, (bf16*)dx, dw, db, rows, d, scale);
   });
@@ -968,6 +976,7 @@ extern "C" int ob_rmsnorm_rope_bwd(const void* dy, const void* x, const void* w,
     using Sh = decltype(shape);
     const int rpb = NORM_THREADS / Sh::TPR;
     constexpr auto kernel = rmsnorm_rope_bwd_kernel<Sh::TPR, Sh::VPT>;
+    allow_smem<kernel>(smem, Sh::TPR * Sh::VPT * 16 * sizeof(float));
     kernel<<<resident_grid<kernel>((rows + rpb - 1) / rpb, smem), NORM_THREADS, smem, stream>>>(
         (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (bf16*)dx, dw, cos_t, sin_t, rows, d, hd, heads, ld_dy,
         ld_x, ld_dx, S, dw_scale);

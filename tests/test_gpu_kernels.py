@@ -579,7 +579,8 @@ def test_rmsnorm_thread_layouts(K, rows, d):
 
 
 @pytest.mark.parametrize("rows,d,bias", [(300, 512, True), (70, 4096, True), (33, 8192, False), (257, 128, True),
-                                           (65, 2048, True)])
+                                           (65, 2048, True), (35, 768, True), (301, 1024, True), (41, 5120, True),
+                                           (40, 6144, True), (40, 6144, False)])
 def test_layernorm(K, rows, d, bias):
     dev = "cuda"
     torch.manual_seed(8)
@@ -725,6 +726,26 @@ def test_fused_rmsnorm_rope_matches_the_two_kernels_and_the_fp32_reference(K, B,
     K.rmsnorm_rope_bwd(dy, x, w, rstd, dx, cos, sin, rows=rows, d=d, hd=hd, heads=heads, seq_len=S, dw=dw, dw_scale=0.5,
                        ld_dy=width, ld_x=width, ld_dx=width)
     assert rel_err(dx, gx) < 1e-2 and rel_err(dw, 0.5 * gw) < 1e-2
+    _check_status()
+
+
+@pytest.mark.parametrize("n", [95, 96, 128])   # 96: just over 48 KB of shared memory with the static part; 128: the widest
+def test_fused_rmsnorm_rope_backward_of_wide_rows(K, n):
+    S, hd, rows = 9, 128, 18
+    d = n * hd
+    torch.manual_seed(10)
+    x, dy = (torch.randn(rows, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    w = (torch.randn(d, device="cuda") * 0.1 + 1).to(torch.bfloat16)
+    cos, sin = ref.rope_tables(S, hd, 500000.0, device="cuda")
+    xf, wf = x.float().requires_grad_(True), w.float().requires_grad_(True)
+    want = ref.apply_rope(ref.rms_norm(xf, wf, 1e-5).view(2, S, n, hd), cos, sin)
+    gx, gw = torch.autograd.grad(want, (xf, wf), dy.float().view(2, S, n, hd))
+    y, rstd = torch.empty_like(x), torch.empty(rows, device="cuda")
+    K.rmsnorm_rope_fwd(x, w, y, rstd, cos, sin, rows=rows, d=d, hd=hd, heads=1, seq_len=S, eps=1e-5)
+    assert rel_err(y.view(2, S, n, hd), want) < 4e-3   # one bf16 rounding, 2^-9 at most
+    dx, dw = torch.empty_like(x), torch.zeros(d, device="cuda")
+    K.rmsnorm_rope_bwd(dy, x, w, rstd, dx, cos, sin, rows=rows, d=d, hd=hd, heads=1, seq_len=S, dw=dw)
+    assert rel_err(dx, gx) < 4e-3 and rel_err(dw, gw) < 1e-5
     _check_status()
 
 
