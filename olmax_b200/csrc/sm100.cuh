@@ -486,13 +486,24 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
 // gated-MLP activations, shared by the GEMM's epilogue (forward) and the element-wise kernels (which rebuild in backward
 // the value that forward rounded): x * sigmoid(z) with z = x (SiLU) or 2 sqrt(2 / pi) (x + 0.044715 x^3) (GELU, tanh form:
 // 0.5 x (1 + tanh(z / 2)) without its cancellation for negative x).  sigmoid = 1 / (1 + 2^t), t = -z * log2(e): two
-// hardware approximations of 1-2 ulp and no branch.
+// hardware approximations of 1-2 ulp and no branch.  The reciprocal is taken of (1 + 2^t) / 4: of 1 + 2^t it would be flushed
+// to zero from 2^126 on, where x * sigmoid is still a normal number (SiLU at -87.5, -88 and -88.5).
 // ---------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float sigmoid_exp2(float t) {
-  float e, r;
+__device__ __forceinline__ float ex2_approx(float t) {
+  float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return e;
+}
+__device__ __forceinline__ float rcp_approx(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   return r;
+}
+__device__ __forceinline__ float sigmoid_exp2(float t) { return rcp_approx(fmaf(ex2_approx(t), 0.25f, 0.25f)) * 0.25f; }
+__device__ __forceinline__ float2 sigmoid_exp2(float2 t) {
+  const float2 quarter = make_float2(0.25f, 0.25f);
+  const float2 d = fma2(make_float2(ex2_approx(t.x), ex2_approx(t.y)), quarter, quarter);
+  return mul2(make_float2(rcp_approx(d.x), rcp_approx(d.y)), quarter);
 }
 constexpr float SILU_T = -1.4426950408889634f;                       // t = x * SILU_T
 constexpr float GELU_T1 = -2.f * 0.7978845608028654f * 1.4426950408889634f, GELU_T3 = GELU_T1 * 0.044715f;
@@ -500,12 +511,10 @@ __device__ __forceinline__ float silu_sigmoid(float x) { return sigmoid_exp2(x *
 __device__ __forceinline__ float gelu_sigmoid(float x) { return sigmoid_exp2(x * fmaf(x * x, GELU_T3, GELU_T1)); }
 // the same for two values, with two-wide instructions where they exist (bit for bit the scalar results)
 __device__ __forceinline__ float2 silu_sigmoid2(float2 x) {
-  const float2 t = mul2(x, make_float2(SILU_T, SILU_T));
-  return make_float2(sigmoid_exp2(t.x), sigmoid_exp2(t.y));
+  return sigmoid_exp2(mul2(x, make_float2(SILU_T, SILU_T)));
 }
 __device__ __forceinline__ float2 gelu_sigmoid2(float2 x) {
-  const float2 t = mul2(x, fma2(mul2(x, x), make_float2(GELU_T3, GELU_T3), make_float2(GELU_T1, GELU_T1)));
-  return make_float2(sigmoid_exp2(t.x), sigmoid_exp2(t.y));
+  return sigmoid_exp2(mul2(x, fma2(mul2(x, x), make_float2(GELU_T3, GELU_T3), make_float2(GELU_T1, GELU_T1))));
 }
 
 }  // namespace ob

@@ -693,6 +693,37 @@ def test_rope_and_glu(K):
     _check_status()
 
 
+@pytest.mark.parametrize("gelu,lowest", [(False, -88.5), (True, -10.0)])   # from where 2^t of the sigmoid's denominator is finite
+def test_gated_activations_of_every_bf16_value(K, gelu, lowest):
+    """act(g) and its gradient against 64 bits for every bf16 value, through the element-wise kernels and the GEMM's epilogue.
+    fp32 error: 3 roundings of t <= 128 and a few ulp, below 3e-5 relative; then one bf16 rounding, 2^-8 at most."""
+    g = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    g = g[(g >= lowest) & (g < 1e9)]
+    g = torch.cat([g, g.new_zeros(-g.numel() % 8)])
+    one, a, dg, du, a2 = (torch.ones_like(g) for _ in range(5))
+    K.glu_fwd(g, one, a, gelu)
+    K.glu_bwd(g, one, one, dg, du, a2, gelu)
+    x = g.double().requires_grad_(True)
+    want = x * torch.sigmoid(2 * math.sqrt(2 / math.pi) * (x + 0.044715 * x ** 3) if gelu else x)
+    (grad,) = torch.autograd.grad(want.sum(), x)
+    want = want.detach()
+    tiny = 2.0 ** -133   # spacing of bf16 below 2^-126
+    assert ((a.double() - want).abs() <= (2.0 ** -8 + 3e-5) * want.abs() + tiny).all()
+    # (the gradient crosses zero: its terms are 1 in size there)
+    assert ((dg.double() - grad).abs() <= (2.0 ** -8 + 3e-5) * grad.abs() + 2.0 ** -21 * (x > -4) + tiny).all()
+    assert torch.equal(a2, a) and torch.equal(du, a)
+    # g and u as one-hot products
+    M, h, Kd = g.numel(), 128, 64
+    rows = torch.zeros(M, Kd, device="cuda", dtype=torch.bfloat16)
+    rows[:, 0], rows[:, 1] = g, 1
+    w1, w2 = (torch.zeros(h, Kd, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    w1[:, 0], w2[:, 1] = 1, 1
+    out = torch.empty(M, h, device="cuda", dtype=torch.bfloat16)
+    K.gemm(rows, w1, out, M, h, Kd, b2=w2, epi=K.EPI_GEGLU if gelu else K.EPI_SWIGLU)
+    assert torch.equal(out, a[:, None].expand(M, h))
+    _check_status()
+
+
 @pytest.mark.parametrize("B,S,n,hd,head_wise", [
     (2, 96, 32, 128, False),     # norm over the whole 4096-wide projection (256 pairs: one per thread)
     (2, 96, 8, 128, False),      # 1024-wide k projection of a grouped-query model
