@@ -191,8 +191,8 @@ def test_gemm_segmented_operands(K, M, Kd, widths):
     dw = torch.zeros(N, Kd, device="cuda")
     K.gemm(dys[0], x, dw, N, Kd, M, a_mn=True, b_mn=True, epi=K.EPI_F32_ACC, alpha=0.5, seg=K.SEG_A_M, seg_rest=dys[1:])
     assert rel_err(dw, 0.5 * dcat.t() @ x.float()) < 2e-5
-    with pytest.raises(Exception):   # a boundary inside a tile
-        K.gemm(x, w[:192], ys[0][:, :64], M, 192, Kd, seg=K.SEG_C_N, seg_rest=[ys[1]])
+    with pytest.raises(K.KernelError, match="multiples of 128"):   # a boundary inside a tile
+        K.gemm(x, w, ys[0][:, :64], M, 64 + widths[1], Kd, seg=K.SEG_C_N, seg_rest=[ys[1]])
     _check_status()
 
 

@@ -77,6 +77,86 @@ def test_model_matches_cpu_restatement(name):
         assert ((a - b).norm() / (a.norm() + 1e-20)).item() < 8e-2, n
 
 
+@pytest.mark.parametrize("used", ["all", "last"])   # outputs that carry a gradient
+@pytest.mark.parametrize("widths,bias,joined", [
+    ((128, 128), False, True),
+    ((384, 128, 256), False, True),
+    ((136, 128), False, False),       # rows that are no whole tiles
+    ((128, 136, 128), False, False),
+    ((128, 128), True, False),        # the biases lie between the weights
+])
+def test_linears_of_one_input_joined_and_apart(widths, bias, joined, used):
+    """``linear_group`` over handles of a parameter store: outputs, dx and the whole flat gradient buffer (the weight that
+    follows the group too, which has none) as from calls one by one."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from olmax_b200.nn.linear import Linear, linear_group
+    from olmax_b200.nn.module import Module, build_module, current_build_context
+    from olmax_b200.ops import _lib, functional as F
+    from olmax_b200.testing import rel_err
+
+    class Group(Module):
+        def __init__(self):
+            super().__init__()
+            self.mods = torch.nn.ModuleList()
+            for i, n in enumerate((*widths, 128)):
+                with current_build_context().scope(f"p{i}"):
+                    self.mods.append(Linear(256, n, bias=bias))
+
+    group = build_module(Group, seed=3, mesh_resource=MeshResource.FSDP(1), device=torch.device("cuda"))
+    mods = list(group.mods)[: len(widths)]
+    assert F._joined([m.weight for m in mods]) == joined
+    torch.manual_seed(7)
+    x0 = torch.randn(2, 100, 256, device="cuda", dtype=torch.bfloat16)
+    dys = [torch.randn(2, 100, n, device="cuda", dtype=torch.bfloat16) for n in widths]
+    results = []
+    for run in (lambda x: linear_group(mods, x), lambda x: tuple(m(x) for m in mods)):
+        group.store.set_grad_scale(0.5)
+        group.store.grad.zero_()
+        x = x0.clone().requires_grad_(True)
+        ys = run(x)
+        first = 0 if used == "all" else len(widths) - 1
+        torch.autograd.backward(ys[first:], dys[first:])
+        group.store.finish_backward()
+        results.append((ys, x.grad, group.store.grad.clone()))
+    (ys, dx, grad), (ys1, dx1, grad1) = results
+    for y, y1 in zip(ys, ys1):
+        assert rel_err(y, y1.float()) < 4e-3   # one bf16 rounding each, 2^-9 at most
+    assert rel_err(dx, dx1.float()) < 1e-2     # apart: one bf16 tensor per weight and their bf16 sums
+    assert rel_err(grad, grad1) < 1e-5         # fp32 sums
+    tail = group.mods[-1].weight.meta
+    assert not grad[tail.offset : tail.offset + tail.numel_local].any()
+    _lib.check_status()
+
+
+def test_gated_mlp_joined_and_apart(monkeypatch):
+    """The gated MLP's backward with gate and up as one matrix against the separate GEMMs: dx and every gradient."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from olmax_b200.nn.mlp import GatedMLP
+    from olmax_b200.nn.module import build_module
+    from olmax_b200.ops import _lib, functional as F
+    from olmax_b200.testing import rel_err
+
+    mlp = build_module(lambda: GatedMLP(256, 384), seed=3, mesh_resource=MeshResource.FSDP(1), device=torch.device("cuda"))
+    assert F._joined((mlp.gate_proj.weight, mlp.up_proj.weight))
+    torch.manual_seed(8)
+    x0, dy = (torch.randn(200, 256, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    results = []
+    for joined in (True, False):
+        if not joined:
+            monkeypatch.setattr(F, "_joined", lambda handles: False)
+        mlp.store.set_grad_scale(1.0)
+        mlp.store.grad.zero_()
+        x = x0.clone().requires_grad_(True)
+        mlp(x).backward(dy)
+        mlp.store.finish_backward()
+        results.append((x.grad, mlp.store.grad.clone()))
+    (dx, grad), (dx1, grad1) = results
+    assert rel_err(dx, dx1.float()) < 1e-2 and rel_err(grad, grad1) < 1e-5
+    _lib.check_status()
+
+
 def test_optimizer_step_matches_cpu():
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
