@@ -214,7 +214,11 @@ __device__ __forceinline__ const CUtensorMap* pick_segment(const CUtensorMap* s0
   return s0;
 }
 
-template <bool A_MN, bool B_MN, int CG, int BN>
+// SEG: with a segmented operand.  These are kernels of their own, and the map is fixed in the loop that issues the loads: an
+// issue that comes later after its stage is freed is a load that arrives later.  With the choice of the map in that loop of
+// every kernel, GEMMs without segments took 2-3 % longer (65536 x 3072 x 1024 297 us, now 287; 8192 x 12288 x 4096 541, now
+// 528) and contractions over segments 6 % (8192 x 4096 x 22016 1030, now 969; 966 of one tensor); one branch per map took 10 %.
+template <bool A_MN, bool B_MN, int CG, int BN, bool SEG>
 __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmB2,
                                           const CUtensorMap& tmC, const CUtensorMap& tmS1, const CUtensorMap& tmS2,
                                           const KernelParams& p) {
@@ -306,107 +310,120 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       const int m0 = (mt / p.m_tiles_per_shard) * p.M_s + m_local0;
       const int n_shard = nt / p.n_tiles_per_shard;
       const int n_local0 = (nt % p.n_tiles_per_shard) * p.bn_out;
+      const CUtensorMap* mapA = &tmA;
+      int ma = m0;   // rows in the A operand, from here in its segment (below: ka, likewise)
+      if constexpr (SEG && A_MN)
+        if (p.seg == SEG_A_M) mapA = pick_segment(&tmA, &tmS1, &tmS2, p, ma);
       // k position, advanced without divisions inside the loop
       const int kit_first = (k_begin + k_rot) % k_iters;
       int k_shard = kit_first / p.k_iters_per_shard;
       int k_local = (kit_first % p.k_iters_per_shard) * BK;
       const int k_local_end = p.k_iters_per_shard * BK;
-      for (int i = 0; i < k_count; ++i) {
-        const int k_glob = k_shard * p.Kc_s + k_local;
-        if (!dead) dead = !mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 100);
-        if (p.ag_shards > 0 && !dead) {
-          int ag_s, ag_b;
-          if (p.ag_on_a) {
-            ag_s = mt / p.m_tiles_per_shard;
-            ag_b = min(m_local0, p.M_s - 1) / AG_BLOCK_ROWS;
-          } else if (B_MN) {
-            ag_s = k_shard;
-            ag_b = k_local / AG_BLOCK_ROWS;
-          } else {
-            ag_s = n_shard;
-            ag_b = n_local0 / AG_BLOCK_ROWS;
-          }
-          const int ag_idx = ((ag_s - p.ag_rank + p.ag_shards) % p.ag_shards) * p.ag_blocks + ag_b;
-          if (ag_idx > ag_ready_idx) {
-            dead = !ag_wait(p, ag_s, ag_b, abort_flag);
-            ag_ready_idx = ag_idx;
+      for (int i = 0; i < k_count;) {   // once; with a segmented contraction once per segment
+        int k_stop = k_count, k_seg = 0;   // the iterations up to which the segment lasts, and where it begins
+        if constexpr (SEG && !A_MN) {
+          if (p.seg == SEG_A_K) {
+            int ka = k_local;
+            mapA = pick_segment(&tmA, &tmS1, &tmS2, p, ka);
+            k_seg = k_local - ka;
+            const int k_end = k_local < p.seg_end[0] ? p.seg_end[0] : p.seg_end[1];
+            if (k_local < k_end) k_stop = min(k_count, i + (k_end - k_local) / BK);
           }
         }
-        const CUtensorMap* mapA = &tmA;
-        int ka = k_glob, ma = m0;   // position in the A operand (segment)
-        if (p.seg == SEG_A_K) mapA = pick_segment(&tmA, &tmS1, &tmS2, p, ka);
-        if (p.seg == SEG_A_M) mapA = pick_segment(&tmA, &tmS1, &tmS2, p, ma);
-        uint8_t* sa = smem + stage * STAGE_BYTES;
-        uint8_t* sb = sa + A_STAGE_BYTES;
-        if (leader && !dead) {
-          if (CG == 1) {
-            mbar_arrive_expect_tx(&full_bar[stage], STAGE_BYTES);
-            if (A_MN) {
-              if (p.a_single) {
-                // one 4-D box: (64 elements, 64 k-rows, 2 column blocks): lands as [block][k][128 B]
-                tma_load_4d(sa, mapA, &full_bar[stage], 0, ka, ma >> 6, 0);
-              } else {
-                tma_load_3d(sa, mapA, &full_bar[stage], ma, ka, 0);
-                tma_load_3d(sa + MN_BLOCK_BYTES, mapA, &full_bar[stage], ma + 64, ka, 0);
-              }
+        for (; i < k_stop; ++i) {
+          const int k_glob = k_shard * p.Kc_s + k_local;
+          const int ka = k_glob - k_seg;
+          if (!dead) dead = !mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 100);
+          if (p.ag_shards > 0 && !dead) {
+            int ag_s, ag_b;
+            if (p.ag_on_a) {
+              ag_s = mt / p.m_tiles_per_shard;
+              ag_b = min(m_local0, p.M_s - 1) / AG_BLOCK_ROWS;
+            } else if (B_MN) {
+              ag_s = k_shard;
+              ag_b = k_local / AG_BLOCK_ROWS;
             } else {
-              tma_load_3d(sa, mapA, &full_bar[stage], ka, ma, 0);
+              ag_s = n_shard;
+              ag_b = n_local0 / AG_BLOCK_ROWS;
             }
-            if (B_MN) {
-              // dims (N, Kc_s, k_shards): BN / 64 64-wide blocks along N
-              const int n0 = n_local0;  // MN-major B is never N-sharded
-              if (p.b_single) {
-                tma_load_4d(sb, &tmB, &full_bar[stage], 0, k_local, n0 >> 6, k_shard);
+            const int ag_idx = ((ag_s - p.ag_rank + p.ag_shards) % p.ag_shards) * p.ag_blocks + ag_b;
+            if (ag_idx > ag_ready_idx) {
+              dead = !ag_wait(p, ag_s, ag_b, abort_flag);
+              ag_ready_idx = ag_idx;
+            }
+          }
+          uint8_t* sa = smem + stage * STAGE_BYTES;
+          uint8_t* sb = sa + A_STAGE_BYTES;
+          if (leader && !dead) {
+            if (CG == 1) {
+              mbar_arrive_expect_tx(&full_bar[stage], STAGE_BYTES);
+              if (A_MN) {
+                if (p.a_single) {
+                  // one 4-D box: (64 elements, 64 k-rows, 2 column blocks): lands as [block][k][128 B]
+                  tma_load_4d(sa, mapA, &full_bar[stage], 0, ka, ma >> 6, 0);
+                } else {
+                  tma_load_3d(sa, mapA, &full_bar[stage], ma, ka, 0);
+                  tma_load_3d(sa + MN_BLOCK_BYTES, mapA, &full_bar[stage], ma + 64, ka, 0);
+                }
               } else {
+                tma_load_3d(sa, mapA, &full_bar[stage], ka, ma, 0);
+              }
+              if (B_MN) {
+                // dims (N, Kc_s, k_shards): BN / 64 64-wide blocks along N
+                const int n0 = n_local0;  // MN-major B is never N-sharded
+                if (p.b_single) {
+                  tma_load_4d(sb, &tmB, &full_bar[stage], 0, k_local, n0 >> 6, k_shard);
+                } else {
 #pragma unroll
-                for (int j = 0; j < BN / 64; ++j)
-                  tma_load_3d(sb + j * MN_BLOCK_BYTES, &tmB, &full_bar[stage], n0 + j * 64, k_local, k_shard);
-              }
-            } else if (glu) {
-              tma_load_3d(sb, &tmB, &full_bar[stage], k_glob, n_local0, n_shard);
-              tma_load_3d(sb + G::B_STAGE_BYTES / 2, &tmB2, &full_bar[stage], k_glob, n_local0, n_shard);
-            } else {
-              tma_load_3d(sb, &tmB, &full_bar[stage], k_glob, n_local0, n_shard);
-            }
-          } else {
-            // CTA pair: both CTAs' copies complete on the leader's barrier, which expects the bytes of both
-            const uint32_t fb = bars_leader + (uint32_t)stage * 8u;
-            if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
-            if (A_MN) {
-              if (p.a_single) {
-                tma_load_4d_pair(sa, mapA, fb, 0, ka, ma >> 6, 0);
+                  for (int j = 0; j < BN / 64; ++j)
+                    tma_load_3d(sb + j * MN_BLOCK_BYTES, &tmB, &full_bar[stage], n0 + j * 64, k_local, k_shard);
+                }
+              } else if (glu) {
+                tma_load_3d(sb, &tmB, &full_bar[stage], k_glob, n_local0, n_shard);
+                tma_load_3d(sb + G::B_STAGE_BYTES / 2, &tmB2, &full_bar[stage], k_glob, n_local0, n_shard);
               } else {
-                tma_load_3d_pair(sa, mapA, fb, ma, ka, 0);
-                tma_load_3d_pair(sa + MN_BLOCK_BYTES, mapA, fb, ma + 64, ka, 0);
+                tma_load_3d(sb, &tmB, &full_bar[stage], k_glob, n_local0, n_shard);
               }
             } else {
-              tma_load_3d_pair(sa, mapA, fb, ka, ma, 0);
-            }
-            if (B_MN) {
-              const int n0 = n_local0 + cta_rank * BNL;   // this CTA's half of the tile's columns: two 64-wide blocks
-              if (p.b_single) {
-                tma_load_4d_pair(sb, &tmB, fb, 0, k_local, n0 >> 6, k_shard);
+              // CTA pair: both CTAs' copies complete on the leader's barrier, which expects the bytes of both
+              const uint32_t fb = bars_leader + (uint32_t)stage * 8u;
+              if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
+              if (A_MN) {
+                if (p.a_single) {
+                  tma_load_4d_pair(sa, mapA, fb, 0, ka, ma >> 6, 0);
+                } else {
+                  tma_load_3d_pair(sa, mapA, fb, ma, ka, 0);
+                  tma_load_3d_pair(sa + MN_BLOCK_BYTES, mapA, fb, ma + 64, ka, 0);
+                }
               } else {
+                tma_load_3d_pair(sa, mapA, fb, ka, ma, 0);
+              }
+              if (B_MN) {
+                const int n0 = n_local0 + cta_rank * BNL;   // this CTA's half of the tile's columns: two 64-wide blocks
+                if (p.b_single) {
+                  tma_load_4d_pair(sb, &tmB, fb, 0, k_local, n0 >> 6, k_shard);
+                } else {
 #pragma unroll
-                for (int j = 0; j < BNL / 64; ++j)
-                  tma_load_3d_pair(sb + j * MN_BLOCK_BYTES, &tmB, fb, n0 + j * 64, k_local, k_shard);
+                  for (int j = 0; j < BNL / 64; ++j)
+                    tma_load_3d_pair(sb + j * MN_BLOCK_BYTES, &tmB, fb, n0 + j * 64, k_local, k_shard);
+                }
+              } else if (glu) {
+                // accumulator columns [0,128) = gate (leader's B half), [128,256) = up (peer's B half)
+                tma_load_3d_pair(sb, cta_rank == 0 ? &tmB : &tmB2, fb, k_glob, n_local0, n_shard);
+              } else {
+                tma_load_3d_pair(sb, &tmB, fb, k_glob, n_local0 + cta_rank * BNL, n_shard);
               }
-            } else if (glu) {
-              // accumulator columns [0,128) = gate (leader's B half), [128,256) = up (peer's B half)
-              tma_load_3d_pair(sb, cta_rank == 0 ? &tmB : &tmB2, fb, k_glob, n_local0, n_shard);
-            } else {
-              tma_load_3d_pair(sb, &tmB, fb, k_glob, n_local0 + cta_rank * BNL, n_shard);
             }
           }
-        }
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        k_local += BK;
-        if (k_local == k_local_end) {
-          k_local = 0;
-          if (++k_shard == p.k_shards) k_shard = 0;
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+          k_local += BK;
+          if (k_local == k_local_end) {
+            k_local = 0;
+            if (++k_shard == p.k_shards) k_shard = 0;
+          }
         }
       }
     }
@@ -611,6 +628,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         for (int c0 = 0; c0 < BN; c0 += cols, ++chunk) {
           if (c0 >= n_valid) break;
           uint8_t* stage_buf = epi_smem + (chunk & 1) * EPI_STAGE_BYTES;
+          const CUtensorMap* mapC = &tmC;
+          int out_col = n_glob0 + c0;   // in the output (segment)
+          if constexpr (SEG)
+            if (p.seg == SEG_C_N) mapC = pick_segment(&tmC, &tmS1, &tmS2, p, out_col);
           if (store_thread && p.tma_epi == 1) tma_store_wait_read<1>();   // the store that last read this buffer is done
           asm volatile("bar.sync 1, 128;" ::: "memory");
           uint32_t r[32], r2[32];
@@ -657,11 +678,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             if (store_thread) {
               if (m_valid > 0) {   // a pair tile's second half may lie wholly below the shard
                 if (p.epi == EPI_F32_ACC) tma_reduce_add_3d(&tmC, stage_buf, n_glob0 + c0, out_row, out_z);
-                else {
-                  int n = n_glob0 + c0;
-                  const CUtensorMap* mapC = p.seg == SEG_C_N ? pick_segment(&tmC, &tmS1, &tmS2, p, n) : &tmC;
-                  tma_store_3d(mapC, stage_buf, n, out_row, out_z);
-                }
+                else tma_store_3d(mapC, stage_buf, out_col, out_row, out_z);
               }
               tma_store_commit();
             }
@@ -855,22 +872,22 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   }
 }
 
-template <bool A_MN, bool B_MN, int BN>
+template <bool A_MN, bool B_MN, int BN, bool SEG>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                      const __grid_constant__ CUtensorMap tmS1, const __grid_constant__ CUtensorMap tmS2, const KernelParams p) {
-  gemm_body<A_MN, B_MN, 1, BN>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
+  gemm_body<A_MN, B_MN, 1, BN, SEG>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
 }
 
 // The CTA-pair variant: the grid is a whole number of 2-CTA clusters.
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool SEG>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                           const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                           const __grid_constant__ CUtensorMap tmS1, const __grid_constant__ CUtensorMap tmS2,
                           const KernelParams p) {
-  gemm_body<A_MN, B_MN, 2, BN_WIDE>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
+  gemm_body<A_MN, B_MN, 2, BN_WIDE, SEG>(tmA, tmB, tmB2, tmC, tmS1, tmS2, p);
 }
 
 constexpr int MAX_DEVICES = 64;
@@ -881,7 +898,7 @@ struct Maps {
   CUtensorMap A, B, B2, C, S1, S2;
 };
 
-template <bool A_MN, bool B_MN, int CG, int BN>
+template <bool A_MN, bool B_MN, int CG, int BN, bool SEG>
 static int launch(const Maps& m, const KernelParams& kp, int grid, cudaStream_t stream) {
   // the shared-memory opt-in is a per-device attribute of the function
   static bool attr_set[MAX_DEVICES] = {};
@@ -891,25 +908,31 @@ static int launch(const Maps& m, const KernelParams& kp, int grid, cudaStream_t 
   constexpr int smem = Geo<CG, BN>::SMEM_BYTES;
   if constexpr (CG == 2) {
     if (!attr_set[dev]) {
-      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<A_MN, B_MN, SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       attr_set[dev] = true;
     }
-    gemm_bf16_pair_kernel<A_MN, B_MN><<<grid, GEMM_THREADS, smem, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
+    gemm_bf16_pair_kernel<A_MN, B_MN, SEG><<<grid, GEMM_THREADS, smem, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
   } else {
     if (!attr_set[dev]) {
-      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      OB_CUDA_OK(cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN, SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       attr_set[dev] = true;
     }
-    gemm_bf16_kernel<A_MN, B_MN, BN><<<grid, GEMM_THREADS, smem, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
+    gemm_bf16_kernel<A_MN, B_MN, BN, SEG><<<grid, GEMM_THREADS, smem, stream>>>(m.A, m.B, m.B2, m.C, m.S1, m.S2, kp);
   }
   OB_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-template <int CG, int BN>
+template <int CG, int BN, bool SEG>
 static int launch_layout(bool a_mn, bool b_mn, const Maps& m, const KernelParams& kp, int grid, cudaStream_t stream) {
-  if (a_mn) return b_mn ? launch<true, true, CG, BN>(m, kp, grid, stream) : launch<true, false, CG, BN>(m, kp, grid, stream);
-  return b_mn ? launch<false, true, CG, BN>(m, kp, grid, stream) : launch<false, false, CG, BN>(m, kp, grid, stream);
+  if (a_mn)
+    return b_mn ? launch<true, true, CG, BN, SEG>(m, kp, grid, stream) : launch<true, false, CG, BN, SEG>(m, kp, grid, stream);
+  return b_mn ? launch<false, true, CG, BN, SEG>(m, kp, grid, stream) : launch<false, false, CG, BN, SEG>(m, kp, grid, stream);
+}
+template <int CG, int BN>
+static int launch_tiles(bool a_mn, bool b_mn, const Maps& m, const KernelParams& kp, int grid, cudaStream_t stream) {
+  return kp.seg != SEG_NONE ? launch_layout<CG, BN, true>(a_mn, b_mn, m, kp, grid, stream)
+                            : launch_layout<CG, BN, false>(a_mn, b_mn, m, kp, grid, stream);
 }
 
 // 1: force single-CTA tiles, 2: force CTA pairs, 0: choose per problem (OLMAX_B200_GEMM_CTA_GROUP)
@@ -1223,9 +1246,9 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     kp.tma_epi = 2;
   if (a->c_shards != nullptr && a->epi == EPI_BF16_ACC && kp.tma_epi != 2)
     OB_FAIL(-18, "EPI_BF16_ACC towards c_shards needs the staged epilogue (16-byte aligned rows, local partial in c)");
-  if (CG == 2) return launch_layout<2, BN_WIDE>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
-  if (BN == BN_NARROW) return launch_layout<1, BN_NARROW>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
-  return launch_layout<1, BN_WIDE>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
+  if (CG == 2) return launch_tiles<2, BN_WIDE>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
+  if (BN == BN_NARROW) return launch_tiles<1, BN_NARROW>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
+  return launch_tiles<1, BN_WIDE>(a->a_mn != 0, a->b_mn != 0, maps, kp, grid, stream);
 }
 
 extern "C" const char* ob_last_error() { return ob::last_error_buf(); }
