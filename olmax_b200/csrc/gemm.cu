@@ -946,7 +946,8 @@ static int cta_group_override() {
 }
 // Cut `tiles` tiles (fewer than workers) of k_iters iterations into `split` k slices each, dealt to the workers in rounds:
 // the split with the shortest schedule, in iterations.  A slice has at least 16 iterations; every round costs about one
-// more for its epilogue (the reduce-add of an fp32 tile runs under the next slice), the last of them eight.
+// more for its epilogue (the reduce-add of an fp32 tile runs under the next slice), the last of them eight.  More slices have
+// to promise 5 %: the model is no closer than that (5632 x 1024 x 65536 in 21 slices, 3 % ahead by it, 522 us; in 5 519).
 struct Split {
   int split;
   double cost;
@@ -956,7 +957,7 @@ static Split best_split(int tiles, int workers, int k_iters) {
   for (int s = 2; s <= 64 && k_iters / s >= 16; ++s) {
     const int rounds = (tiles * s + workers - 1) / workers;
     const double cost = rounds * ((double)k_iters / s + 1.0) + 8.0;
-    if (cost < 0.98 * best.cost) best = Split{s, cost};
+    if (cost < 0.95 * best.cost) best = Split{s, cost};
   }
   return best;
 }
