@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 
 // dx = rstd * (w*dy - xhat * mean(w*dy*xhat)) (+ dsum);  dw += sum_rows dy * xhat  (fp32 atomics, accumulating)
 // (Next row group fetched before the current one is reduced, as in the forward kernel.  DSUM, with a residual gradient: that
-// row too; read after the row's barriers it cost [65536, 1024] 127 us against 111, [5560, 5120] 70 against 59.  The rows in
+// row too; read after the row's barriers it cost [65536, 1024] 123 us against 109, [5560, 5120] 68 against 55.  The rows in
 // flight then need the registers of one block per SM: [8192, 4096] 64 -> 57 us, 67 with the limit of the plain form, which
 // in turn would lose 45 -> 51 us with this one's.)
 template <int TPR, int VPT, bool DSUM>

@@ -19,8 +19,8 @@
 // 2560 cycles of tensor work and about 1024 cycles of MUFU work for the exponentials).
 //
 // All kernels of the backward, before (P and dS through shared memory, dQ drained by the compute warps, every MMA waiting for
-// the previous stage of the same tile) and now: B 2, S 4096, H 32 causal 1058 -> 723 us; B 3, S 1515, H 40 / 8 464 -> 238 us;
-// B 1, S 8192, H 32 / 16, window 4096, soft-cap 1858 -> 1080 us.
+// the previous stage of the same tile) and now: B 2, S 4096, H 32 causal 1058 -> 730 us; B 3, S 1515, H 40 / 8 464 -> 238 us;
+// B 1, S 8192, H 32 / 16, window 4096, soft-cap 1858 -> 1078 us (one GPU; others at other clocks differ by a few per cent).
 //
 // The math is the standard recompute form: P = exp(S - lse), dS = P * (dP - delta) with the softmax scale applied to the
 // sums dQ and dK, delta = rowsum(dO * O) from a pre-pass; a tanh soft-cap multiplies dS by (1 - tanh^2).
@@ -67,7 +67,7 @@ struct Params {
   int Sk, q_off;   // key length; key-axis position of query row 0
   int causal, window;
   int kv_tiles, group;   // key tiles per slice; (batch, kv-head) slices per scheduling group
-  float scale, scale_log2, softcap, scale_over_cap, cap_log2;
+  float scale, scale_log2, scale_over_cap, cap_log2;
   const float* lse;
   const float* delta;
   bf16* dk; long long dk_sb, dk_ss, dk_sh;
@@ -122,10 +122,10 @@ __device__ __forceinline__ Item decode_item(const Params& p, int w) {
 // CAPPED: with a soft-cap.  Its code and registers stay out of the plain kernel, and the other way round.
 // PERSISTENT: the CTA that runs on an SM takes over the items of CTAs that have not started, so that the next item's loads,
 // first scores and dP run under the write-out of dK / dV; else every CTA has its one item.  Without a soft-cap the three
-// kernels of the backward gain by it: B 64, S 1024, H 8 682 -> 618 us (4.5 query tiles per item), B 2, S 4096, H 32
-// 748 -> 723, B 3, S 1515, H 40 / 8 and B 1, S 8192, H 32 / 16, window 4096 unchanged.  With one, the compute warps bound
-// the loop and the longer-lived state costs them: B 1, S 8192, H 32 / 16 1364 -> 1438 us, with window 4096 1058 -> 1075;
-// so the capped kernel keeps one item per CTA.
+// kernels of the backward gain by it (both sides on one GPU each time): B 64, S 1024, H 8 682 -> 618 us (4.5 query tiles
+// per item), B 2, S 4096, H 32 748 -> 723, B 3, S 1515, H 40 / 8 and B 1, S 8192, H 32 / 16, window 4096 unchanged.  With
+// one, the compute warps bound the loop and the longer-lived state costs them: B 1, S 8192, H 32 / 16 1364 -> 1438 us,
+// with window 4096 1058 -> 1075; so the capped kernel keeps one item per CTA.
 template <bool CAPPED>
 __global__ void __launch_bounds__(THREADS, 1)
     flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -868,7 +868,6 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   const float LOG2E = 1.4426950408889634f;
   p.scale = a->scale;
   p.scale_log2 = a->scale * LOG2E;
-  p.softcap = a->softcap;
   p.scale_over_cap = a->softcap > 0.f ? a->scale / a->softcap : 0.f;
   p.cap_log2 = a->softcap * LOG2E;
   p.lse = a->lse;
@@ -879,7 +878,7 @@ static int launch_flash_bwd(const ObAttnArgs* a, float* delta, float* dq_accum, 
   p.kv_tiles = kv_tiles;
   // Few items per SM: the longest loops of all slices first, or the last ones to start set the time.  Many: groups of eight
   // slices, whose Q / dO / dQ (8 MB per 1024 rows, times the heads per kv-head) stay in L2 while their key tiles run.
-  p.group = items <= 4 * 148 ? (int)slices : 8;
+  p.group = items <= 4 * sm_count() ? (int)slices : 8;
   const auto kernel = a->softcap > 0.f ? fa_bwd::flash_bwd_kernel<true> : fa_bwd::flash_bwd_kernel<false>;
   kernel<<<(unsigned)items, fa_bwd::THREADS, fa_bwd::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdq, p);
   OB_CUDA_OK(cudaGetLastError());

@@ -1016,8 +1016,8 @@ extern "C" int ob_gemm_bf16(const ObGemmArgs* a, cudaStream_t stream) {
     if (kp.m_shards > 1 && M_s <= BM) CG = 1;
     // 128 x 64 tiles, where all of them run at once and most pairs would have no 256 x 256 tile.  Their k-blocks come at the
     // same pace (about 280 ns, bound by the latency of the loads through eight stages), but they start and drain sooner:
-    // 328 x 1024 x 2816 20.5 us against 26.7 with 128 x 256 single-CTA tiles, 1000 x 1024 x 5632 35 against 43, 1024 x
-    // 512 x 512 12.3 against 14.3.  In more than one wave they lose (2048 x 1024 x 50304: 533 us against 240 with pairs),
+    // 328 x 1024 x 2816 22.6 us against 26.6 with 128 x 256 single-CTA tiles, 1000 x 1024 x 5632 37 against 42, 1024 x
+    // 512 x 512 12.3 against 14.3.  In more than one wave they lose (2048 x 1024 x 50304: 533 us against 242 with pairs),
     // and to k slices on pairs where the contraction is long enough to be cut.
     if (!sharded && !glu && tiles(BM, BN_WIDE) <= cap / 2 && tiles(BM, BN_NARROW) <= cap &&
         !(split_ok && best_split((int)pair_tiles, cap / 2, k_iters_total).split > 1)) {

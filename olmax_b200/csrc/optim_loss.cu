@@ -15,7 +15,7 @@
 namespace ob {
 
 constexpr int CE_THREADS = 512;
-constexpr int CE_CACHE = 48 * 1024 / 4;   // logits of a row kept in shared memory: four blocks per SM
+constexpr int CE_CACHE = 48 * 1024 / 4;   // logits of a row kept in shared memory
 
 __device__ __forceinline__ float tanh_fast(float x) {
   float y;
@@ -36,12 +36,12 @@ __device__ __forceinline__ MaxSum combine(MaxSum a, MaxSum b) {
 //   stats[0] += sum over valid rows of loss;  stats[1] += sum over valid rows of lse^2 (z-loss numerator)
 //   inv_count: device float, 1 / (number of valid labels in the whole batch)
 // Bound by HBM.  The row is read twice (statistics, gradient): its first `cached` elements wait in shared memory for the
-// second pass, which reads the rest from its end backwards, where most of it is still in L2.  Four blocks per SM overlap one
-// another's passes.  Each thread has CE_UNROLL 16-byte loads in flight and takes the maximum of the batch before its
+// second pass, which reads the rest from its end backwards, where most of it is still in L2.  Three blocks per SM (what
+// 40 registers per thread allow) overlap one another's passes.  Each thread has CE_UNROLL 16-byte loads in flight and takes the maximum of the batch before its
 // exponentials, which then do not wait for one another.  2048 rows of 50304 / 100352 / 256000 (soft-cap) logits with the
 // gradient: 186 / 352 / 908 us with one load in flight and the row read twice from its start; 164 / 316 / 815 with the
-// batches alone, 152 / 303 / 803 backwards, 143 / 291 / 792 with 48 KB of the row kept (96 KB, two blocks per SM: 158 / 305 /
-// 856).  The loss alone: 109 / 184 / 447 -> 94 / 158 / 367 us.
+// batches alone, 152 / 303 / 803 backwards, 143 / 291 / 790 with 48 KB of the row kept (96 KB, two blocks per SM: 158 / 305 /
+// 856).  The loss alone: 109 / 184 / 447 -> 94 / 156 / 367 us.
 constexpr int CE_UNROLL = 4;
 
 __global__ void __launch_bounds__(CE_THREADS)
